@@ -207,3 +207,71 @@ def test_latent_decode_attention_kernel(B, H, ctx, splits):
         ref = torch.softmax(s, -1) @ rows[:, :512]
         err = (o[b].float() - ref).abs().max() / ref.abs().max()
         assert err < 2e-2, (b, float(err))
+
+
+def _hash_u32(x):
+    x &= 0xFFFFFFFF
+    x = ((x ^ (x >> 16)) * 0x7FEB352D) & 0xFFFFFFFF
+    x = ((x ^ (x >> 15)) * 0x846CA68B) & 0xFFFFFFFF
+    return x ^ (x >> 16)
+
+
+def _draw(z, row, t, k, tp, mp, seed, step):
+    """What the sampler picks for one row of (penalised) logits, and its log-probability: the k best by (value, lowest index),
+    top-p and min-p on them, a draw by the counter-based generator."""
+    v, i = torch.sort(z.double(), descending=True, stable=True)
+    n = int((v[:k] > -float("inf")).sum())
+    p = torch.exp((v[:n] - v[0]) / t)
+    share, kept = p / p.sum(), 0
+    cum = 0.0
+    while kept < n and (kept == 0 or (cum < tp and p[kept] >= mp * p[0])):
+        cum += float(share[kept])
+        kept += 1
+    h = _hash_u32((seed & 0xFFFFFFFF) ^ _hash_u32((seed >> 32) + 0x9E3779B9 * (step + 1)) ^ _hash_u32(row))
+    u = ((h >> 8) + 0.5) / 2 ** 24
+    acc = torch.cumsum(p[:kept], 0) / p[:kept].sum()
+    j = min(int((acc < u).sum()), kept - 1)
+    return int(i[j]), float(torch.log_softmax(z.double() / t, -1)[i[j]]), float((acc - u).abs().min())
+
+
+@pytest.mark.parametrize("R,V", [(1, 70), (3, 128256), (40, 128256), (200, 5000), (2, 50257), (1, 8192), (300, 33)])
+@pytest.mark.parametrize("form", ["spread", "ties", "equal", "masked", "sorted"])
+def test_sampler_draws_what_the_oracle_draws(R, V, form):
+    """Rows cut into slices, rows that do not start on 16 bytes, many equal logits, rows of which few tokens are allowed and rows
+    whose best tokens lie side by side: the candidates are the k best by (value, lowest index) in every case."""
+    from easydel_b200.ops import serving as S
+
+    g = torch.Generator(device="cuda").manual_seed(R * 7 + V)
+    dev = "cuda"
+    z = torch.randn(R, V, device=dev, generator=g) * 2.5
+    if form == "ties":
+        z = torch.round(z)
+    elif form == "equal":
+        z = torch.zeros(R, V, device=dev)
+    elif form == "masked":
+        keep = torch.rand(R, V, device=dev, generator=g) < 20 / V
+        keep[:, V // 2] = True
+        z = torch.where(keep, z, -float("inf"))
+    elif form == "sorted":
+        z = z.sort(-1).values
+    for dtype in (torch.bfloat16, torch.float32):
+        logits = z.to(dtype)
+        u = lambda: torch.rand(R, device=dev, generator=g)  # noqa: E731
+        temp, top_p, min_p = 0.5 + u(), 0.5 + 0.5 * u(), 0.1 * u() * (u() < 0.5)
+        top_k = (u() * 70).to(torch.int32)
+        seeds = torch.randint(0, 1 << 40, (R,), device=dev, generator=g)
+        steps = torch.randint(0, 99, (R,), device=dev, generator=g).to(torch.int32)
+        tok, lp = S.sample(logits, temperature=temp, top_k=top_k, top_p=top_p, min_p=min_p, seeds=seeds, steps=steps,
+                           want_logprob=True)
+        zc = logits.float().cpu()
+        for r in range(0, R, max(1, R // 12)):
+            k = int(top_k[r])
+            if k == 1:
+                assert int(tok[r]) == int(zc[r].argmax())
+                continue
+            want, want_lp, margin = _draw(zc[r], r, float(temp[r]), 64 if k <= 0 or k > 64 else k, float(top_p[r]),
+                                          float(min_p[r]), int(seeds[r]), int(steps[r]))
+            if margin < 1e-5:      # the draw falls on a boundary of the fp32 sums
+                continue
+            assert int(tok[r]) == want, (r, k)
+            assert abs(float(lp[r]) - want_lp) < 1e-4 * max(1.0, abs(want_lp))
