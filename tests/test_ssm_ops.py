@@ -239,3 +239,51 @@ def test_chunked_wkv4_matches_the_sequential_reference_with_gradients():
         assert torch.allclose(ssm.wkv4(decay, first, k, v, cu), ssm.wkv4_reference(decay, first, k, v, cu), atol=1e-5)
         assert torch.allclose(ssm.wkv4_chunked(decay, first, k[:7], v[:7], chunk=4),
                               ssm.wkv4_reference(decay, first, k[:7], v[:7]), atol=1e-5)
+
+
+def _tokens_of(lens):
+    return torch.tensor([0] + lens, device="cuda").cumsum(0).to(torch.int32), sum(lens)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("lens", [[8], [1, 7, 8, 9, 0, 16], [130, 3, 257], [5, 1]])
+@pytest.mark.parametrize("DK,DV,H", [(128, 128, 3), (128, 200, 2), (64, 72, 5), (32, 33, 1), (128, 128, 40)])
+@pytest.mark.parametrize("gate", ["head", "channel", "none"])
+def test_delta_rule_in_blocks_matches_the_tokens_one_by_one(lens, DK, DV, H, gate):
+    """Blocks of eight tokens (remainders, empty sequences, column tiles that are not full, plain resets by a gate of minus
+    infinity) against the one-token recurrence in fp32, from a state that is not empty."""
+    torch.manual_seed(5)
+    cu, T = _tokens_of(lens)
+    unit = lambda: torch.nn.functional.normalize(torch.randn(T, H, DK, device="cuda"), dim=-1).to(torch.bfloat16)  # noqa: E731
+    q, k, v = unit(), unit(), torch.randn(T, H, DV, device="cuda").to(torch.bfloat16)
+    g = None if gate == "none" else -3 * torch.rand(*((T, H, DK) if gate == "channel" else (T, H)), device="cuda")
+    if g is not None:
+        g[T // 2] = -float("inf")
+    beta = None if gate == "none" else torch.rand(T, H, device="cuda").to(torch.bfloat16)
+    s1 = torch.randn(len(lens), H, DK, DV, device="cuda")
+    s2 = s1.clone()
+    assert ssm._block_records(T, len(lens), H, q, k) is not None or T < 4 * len(lens)
+    with torch.no_grad():
+        got = ssm.gated_delta_rule(q, k, v, g, beta, None, cu, s1)
+        want = ssm.delta_rule_reference(q.float(), k.float(), v.float(), g, beta, None, cu, s2)
+    # fp32 sums in another order: a few 2^-24 per token; the output is rounded to bf16 (2^-9 of a value)
+    assert (s1 - s2).abs().max() < 1e-5 * s2.abs().max()
+    assert ((got.float() - want).abs() <= 2 ** -8 * want.abs() + 1e-5 * want.abs().max()).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("lens", [[8], [1, 7, 8, 9, 0, 16], [130, 3, 257]])
+@pytest.mark.parametrize("H,P,G,N", [(4, 64, 2, 128), (3, 50, 1, 16), (6, 128, 3, 64), (8, 33, 8, 32), (64, 64, 1, 128)])
+def test_ssd_scan_in_blocks_matches_the_tokens_one_by_one(lens, H, P, G, N):
+    torch.manual_seed(6)
+    cu, T = _tokens_of(lens)
+    bf = lambda *s: torch.randn(*s, device="cuda").to(torch.bfloat16)  # noqa: E731
+    x, dt, B, C = bf(T, H, P), bf(T, H), bf(T, G, N), bf(T, G, N)
+    A, D, bias = -4 * torch.rand(H, device="cuda"), torch.randn(H, device="cuda"), torch.randn(H, device="cuda")
+    s1 = torch.randn(len(lens), H, P, N, device="cuda")
+    s2 = s1.clone()
+    with torch.no_grad():
+        got = ssm.ssd_scan(x, dt, A, B, C, D, bias, True, cu, s1)
+        want = ssm.ssd_scan_reference(x.float(), dt, A, B, C, D, bias, True, cu, s2)
+    assert (s1 - s2).abs().max() < 1e-5 * s2.abs().max()
+    assert ((got.float() - want).abs() <= 2 ** -8 * want.abs() + 1e-5 * want.abs().max()).all()
