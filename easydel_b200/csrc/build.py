@@ -47,7 +47,7 @@ NVCC_FLAGS = [
 
 # Kernels whose job is 32-bit arithmetic (fp32 residual stream, gates and recurrences, attention of fp32 models) are
 # compiled without fast-math.
-PRECISE = frozenset({"stream_ops", "hgrn2", "gdelta", "block_scan", "attention_simt", "latent_ops", "moe_serving"})
+PRECISE = frozenset({"stream_ops", "hgrn2", "gdelta", "block_scan", "chunk_scan", "attention_simt", "latent_ops", "moe_serving"})
 
 # What serving a model family needs, by model type, for a first call on a machine without a built library.
 SERVING_PARTS = {

@@ -1,0 +1,552 @@
+// Token scans of the gated delta rule with a decay per head (Qwen3-Next) and of the Mamba-2 state-space recurrence, sixteen
+// tokens at a time on the tensor cores, in fp32 accuracy. Per head, with a [DK, DV] state S in fp32,
+//
+//   delta rule:  S <- e^{g_t} S ;  r_t = beta_t (v_t - S^T k_t) ;  S <- S + k_t r_t^T ;  o_t = scale S^T q_t
+//   state space: S <- e^{dt_t A} S + B_t (dt_t x_t)^T ;                                  y_t = S^T C_t + D x_t
+//
+// and for a chunk of sixteen tokens behind a state S_0 (decays are exponentials of sums over (i, j], never of differences):
+//
+//   y_j = k_j . S_0 ;  r = T (beta v - eb y),  T = (1 + M)^-1,  M_ji = beta_j e^{g_{i+1} + .. + g_j} k_j . k_i   (i < j)
+//   o_j = es_j q_j . S_0 + sum_{i<=j} P_ji r_i,                 P_ji = scale e^{g_{i+1} + .. + g_j} q_j . k_i
+//   S_16 = e^{g_1 + .. + g_16} S_0 + sum_i e^{g_{i+1} + .. + g_16} k_i r_i^T
+//
+// (state space: r_i = x_i, without y and T; dt_i and D are folded into P and the tails).
+//
+// Accuracy. k, q, B, C, x and v are bf16, so they are exact operands. An fp32 operand enters as three bf16 parts that add up
+// to its 24 bits; products of two such operands take the six pairs of parts that reach 2^-24. Leading parts have accumulators
+// of their own, and the update of the state is summed from zero and then added in fp32, so the state is rounded once per chunk
+// instead of once per token.
+//
+//   * chunk_coef: a warp per (chunk, head) forms the 16 x 16 products (mma.sync on the rows as they lie), the decays, T by
+//     forward substitution, and stores the parts of T and P in the order the scan's lanes read them.
+//   * chunk_scan: the columns of a state never meet. A warp owns 16 of them: S^T lies in the accumulator layout, which is also
+//     the layout of a left operand, so the state never leaves its registers; warps need no exchange. Rows, values and
+//     coefficients come by cp.async, two chunks ahead. What bounds it is the rate of the products: 168 of 16 x 8 x 16 per warp
+//     and chunk for the delta rule with DK = 128, 102 for the state space, at about 20 clocks each, and with one warp per
+//     scheduler the chain y -> T -> P behind them.
+//
+// 5328 + 2864 tokens, 32 heads of 128 x 128: 0.73 ms (eight tokens at a time on the FMA pipe 1.90 ms, one at a time 19.4 ms);
+// 6000 tokens in three sequences, 64 state-space heads of 64 x 128: 0.32 ms (0.74 ms, 4.4 ms). Bytes at the copy rate: 43 and
+// 18 us. A value that is not finite spoils its column for the whole chunk (a zero weight times infinity), not only from its
+// token on.
+// Compiled without fast-math.
+#include "common.cuh"
+
+namespace edl {
+namespace {
+
+constexpr int CS_C = 16;                  // tokens per chunk
+constexpr int CS_WARPS = 4;
+constexpr int CS_THREADS = CS_WARPS * 32;
+constexpr int CS_CT = CS_WARPS * 16;      // columns of a CTA
+constexpr int CS_STAGES = 3;
+
+enum CsMode { CS_DELTA = 0, CS_SSD = 1 };
+
+// Record of a (chunk, head), in bytes: parts of P [3][32 lanes][16] | es 16 | tail 16 | total, pad (floats), and for the delta
+// rule parts of T | beta 16 | eb 16.
+constexpr int CS_P = 0, CS_ES = 1536, CS_TAIL = CS_ES + 64, CS_TOTAL = CS_TAIL + 64, CS_T = CS_TOTAL + 16,
+              CS_BETA = CS_T + 1536, CS_EB = CS_BETA + 64;
+template <int MODE>
+constexpr int cs_rec_bytes() { return MODE == CS_SSD ? CS_T : CS_EB + 64; }
+
+struct CsParams {
+  const __nv_bfloat16 *q, *k, *v;    // [T, G, DK] x 2, [T, H, DV]
+  const float* g;                    // delta: [T, H] log decays, or null
+  const __nv_bfloat16* beta;         // delta: [T, H] or null
+  const __nv_bfloat16* dt;           // state space: [T, H]
+  const float *A, *Dskip, *dt_bias;  // [H]
+  int softplus;
+  const int* cu;
+  int T, B, H, G, DV;
+  float scale;
+  uint8_t* rec;                      // [slots, H, record]
+  float* state;                      // delta [B, H, DK, DV], state space [B, H, DV, DK]; or null
+  __nv_bfloat16* o;                  // [T, H, DV]
+  bool vec_v;                        // values can be fetched 16 bytes at a time
+};
+
+// A chunk's place in the record array: unique and increasing over (sequence, chunk), below T / 16 + B + 1.
+__device__ __forceinline__ int cs_slot(int t, int b) { return t / CS_C + b; }
+
+__device__ __forceinline__ float cs_softplus(float x) { return x > 20.f ? x : log1pf(expf(x)); }
+
+__device__ __forceinline__ void cs_mma(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
+      "{%0, %1, %2, %3};"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void cs_ldmatrix(uint32_t addr, uint32_t (&r)[4]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(addr));
+}
+__device__ __forceinline__ void cs_ldmatrix_trans(uint32_t addr, uint32_t (&r)[4]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(addr));
+}
+// 16 bytes to shared memory, or zeros
+__device__ __forceinline__ void cs_copy16(uint32_t dst, const void* src, bool on) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(on ? 16 : 0) : "memory");
+}
+
+// Two fp32 values as three bf16 pairs that add up to them (24 bits).
+__device__ __forceinline__ void cs_split(float x, float y, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
+  hi = pack_bf16x2(x, y);
+  x -= __uint_as_float(hi << 16);
+  y -= __uint_as_float(hi & 0xffff0000u);
+  mid = pack_bf16x2(x, y);
+  x -= __uint_as_float(mid << 16);
+  y -= __uint_as_float(mid & 0xffff0000u);
+  lo = pack_bf16x2(x, y);
+}
+// A 16 x 16 block in the accumulator layout (two column halves) as the parts of a left operand.
+__device__ __forceinline__ void cs_split_block(const float (&c0)[4], const float (&c1)[4], uint32_t (&a)[3][4]) {
+  cs_split(c0[0], c0[1], a[0][0], a[1][0], a[2][0]);
+  cs_split(c0[2], c0[3], a[0][1], a[1][1], a[2][1]);
+  cs_split(c1[0], c1[1], a[0][2], a[1][2], a[2][2]);
+  cs_split(c1[2], c1[3], a[0][3], a[1][3], a[2][3]);
+}
+
+// ---- coefficients -----------------------------------------------------------------------------------------------------
+template <int MODE, int DK>
+__global__ void __launch_bounds__(128) chunk_coef_kernel(const CsParams p, int heads_per_warp) {
+  constexpr int REC = cs_rec_bytes<MODE>();
+  __shared__ float s_m[4][16][17], s_p[4][16][17], s_g[4][16], s_a[4][16];
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, row = lane >> 2, quad = lane & 3;
+  const int h0 = (blockIdx.y * 4 + w) * heads_per_warp;
+  if (h0 >= p.H) return;
+  const int slot = blockIdx.x;
+  int lo = 0, hi = p.B;                 // the last sequence whose first chunk is not past this slot
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (cs_slot(p.cu[mid], mid) <= slot) lo = mid;
+    else hi = mid;
+  }
+  const int first = p.cu[lo], end = p.cu[lo + 1];
+  const int t0 = first + (slot - cs_slot(first, lo)) * CS_C;
+  if (t0 < first || t0 >= end) return;
+  const int n = min(CS_C, end - t0);
+  const int rows = h0 / (p.H / p.G);
+  // products: a lane takes 16-byte pieces of rows `row` and `row + 8`; which dimension a position of the reduction stands for
+  // does not matter as long as both operands agree
+  float qk[2][4], kk[2][4];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) qk[0][e] = qk[1][e] = kk[0][e] = kk[1][e] = 0.f;
+  auto piece = [&](const __nv_bfloat16* m, int t, int d) {
+    return t < n && d < DK ? *reinterpret_cast<const uint4*>(m + ((long long)(t0 + t) * p.G + rows) * DK + d) : make_uint4(0u, 0u, 0u, 0u);
+  };
+#pragma unroll
+  for (int d = 0; d < DK; d += 32) {
+    const uint4 k0 = piece(p.k, row, d + 8 * quad), k1 = piece(p.k, row + 8, d + 8 * quad);
+    const uint4 q0 = piece(p.q, row, d + 8 * quad), q1 = piece(p.q, row + 8, d + 8 * quad);
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      const uint32_t ka[4] = {half ? k0.z : k0.x, half ? k1.z : k1.x, half ? k0.w : k0.y, half ? k1.w : k1.y};
+      const uint32_t qa[4] = {half ? q0.z : q0.x, half ? q1.z : q1.x, half ? q0.w : q0.y, half ? q1.w : q1.y};
+      cs_mma(qk[0], qa, ka[0], ka[2]);
+      cs_mma(qk[1], qa, ka[1], ka[3]);
+      if (MODE == CS_DELTA) {
+        cs_mma(kk[0], ka, ka[0], ka[2]);
+        cs_mma(kk[1], ka, ka[1], ka[3]);
+      }
+    }
+  }
+  for (int h = h0; h < min(p.H, h0 + heads_per_warp); ++h) {
+    float g = 0.f, a = 0.f;             // log decay; beta or dt
+    if (lane < n) {
+      const long long at = (long long)(t0 + lane) * p.H + h;
+      if (MODE == CS_SSD) {
+        a = __bfloat162float(p.dt[at]) + (p.dt_bias ? p.dt_bias[h] : 0.f);
+        if (p.softplus) a = cs_softplus(a);
+        g = a * p.A[h];
+      } else {
+        a = p.beta ? __bfloat162float(p.beta[at]) : 1.f;
+        if (p.g) g = p.g[at];
+      }
+    }
+    __syncwarp();
+    if (lane < 16) {
+      s_g[w][lane] = g;
+      s_a[w][lane] = a;
+    }
+    __syncwarp();
+    float before = 0.f, after = 0.f;
+#pragma unroll
+    for (int l = 0; l < 16; ++l) {
+      const float x = s_g[w][l];
+      if (l <= lane) before += x;
+      else after += x;
+    }
+    uint8_t* dst = p.rec + ((long long)slot * p.H + h) * REC;
+    if (lane <= 16) {                   // lane 16: the whole chunk
+      const float e = expf(before);
+      if (lane == 16) {
+        *reinterpret_cast<float*>(dst + CS_TOTAL) = e;
+      } else {
+        reinterpret_cast<float*>(dst + CS_ES)[lane] = e * p.scale;
+        reinterpret_cast<float*>(dst + CS_TAIL)[lane] = expf(after) * (MODE == CS_SSD ? a : 1.f);
+        if (MODE == CS_DELTA) {
+          reinterpret_cast<float*>(dst + CS_BETA)[lane] = a;
+          reinterpret_cast<float*>(dst + CS_EB)[lane] = e * a;
+        }
+      }
+    }
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {      // rows j = row, row + 8
+      const int j = row + 8 * half;
+      float d[4] = {0.f, 0.f, 0.f, 0.f}, sum = 0.f;   // decays from columns 2 quad, 2 quad + 1, and eight further
+#pragma unroll
+      for (int l = 15; l >= 0; --l) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          if (l == 2 * quad + (e & 1) + 8 * (e >> 1)) d[e] = sum;
+        if (l <= j) sum += s_g[w][l];
+      }
+      const float aj = s_a[w][j];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int i = 2 * quad + (e & 1) + 8 * (e >> 1);
+        const float f = i <= j ? expf(d[e]) : 0.f;
+        float pv = f * qk[e >> 1][2 * half + (e & 1)];
+        if (MODE == CS_SSD) {
+          pv *= s_a[w][i];
+          if (i == j && p.Dskip) pv += p.Dskip[h];
+        } else {
+          pv *= p.scale;
+          s_m[w][j][i] = i < j ? aj * f * kk[e >> 1][2 * half + (e & 1)] : 0.f;
+        }
+        s_p[w][j][i] = i <= j ? pv : 0.f;
+      }
+    }
+    __syncwarp();
+    float t[16];
+    if (MODE == CS_DELTA) {             // lane c: column c of the inverse of 1 + M
+#pragma unroll
+      for (int j = 0; j < 16; ++j) t[j] = j == (lane & 15) ? 1.f : 0.f;
+#pragma unroll
+      for (int i = 0; i < 15; ++i)
+#pragma unroll
+        for (int j = i + 1; j < 16; ++j) t[j] = fmaf(-s_m[w][j][i], t[i], t[j]);
+      __syncwarp();
+      if (lane < 16)
+#pragma unroll
+        for (int j = 0; j < 16; ++j) s_m[w][j][lane] = t[j];
+      __syncwarp();
+    }
+    // parts in the order of a right operand: for both halves of columns j, rows i = 2 quad, 2 quad + 1 and eight further
+#pragma unroll
+    for (int which = 0; which < (MODE == CS_DELTA ? 2 : 1); ++which) {
+      uint32_t x[3][4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float* m = which ? &s_m[w][row + 8 * (e >> 1)][2 * quad + 8 * (e & 1)] : &s_p[w][row + 8 * (e >> 1)][2 * quad + 8 * (e & 1)];
+        cs_split(m[0], m[1], x[0][e], x[1][e], x[2][e]);
+      }
+#pragma unroll
+      for (int part = 0; part < 3; ++part)
+        *reinterpret_cast<uint4*>(dst + (which ? CS_T : CS_P) + part * 512 + lane * 16) =
+            make_uint4(x[part][0], x[part][1], x[part][2], x[part][3]);
+    }
+  }
+}
+
+// ---- scan -------------------------------------------------------------------------------------------------------------
+template <int MODE, int DK>
+struct CsCfg {
+  static constexpr int PITCH = DK * 2 + 16;              // bytes of a row of k or q
+  static constexpr int VPITCH = CS_CT * 2 + 16;
+  static constexpr int REC = cs_rec_bytes<MODE>();
+  static constexpr int OFF_Q = CS_C * PITCH, OFF_V = 2 * CS_C * PITCH, OFF_R = OFF_V + CS_C * VPITCH;
+  static constexpr int STAGE = OFF_R + REC;
+  static_assert(STAGE % 16 == 0 && CS_STAGES * STAGE <= 48 * 1024, "");
+};
+
+template <int MODE, int DK>
+__global__ void __launch_bounds__(CS_THREADS) chunk_scan_kernel(const CsParams p) {
+  using C = CsCfg<MODE, DK>;
+  constexpr int NT = DK / 8, NK = DK / 16;
+  __shared__ __align__(128) uint8_t smem[CS_STAGES * C::STAGE];
+  const uint32_t base = smem_u32(smem);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, row = lane >> 2, quad = lane & 3;
+  const int h = blockIdx.y, b = blockIdx.z;
+  const int t0 = p.cu[b], t1 = p.cu[b + 1];
+  if (t0 >= t1) return;
+  const int H = p.H, DV = p.DV, rows = h / (p.H / p.G);
+  const int cta_col = blockIdx.x * CS_CT, col = cta_col + warp * 16 + row;    // this lane's columns: col, col + 8
+
+  auto fetch = [&](int tb, int st) {
+    const int n = min(CS_C, t1 - tb);
+    const uint32_t dst = base + st * C::STAGE;
+    for (int i = tid; i < 2 * CS_C * (DK / 8); i += CS_THREADS) {
+      const int which = i / (CS_C * (DK / 8)), t = (i / (DK / 8)) % CS_C, c = i % (DK / 8);
+      const __nv_bfloat16* src = (which ? p.q : p.k) + ((long long)(tb + (t < n ? t : 0)) * p.G + rows) * DK + c * 8;
+      cs_copy16(dst + which * C::OFF_Q + t * C::PITCH + c * 16, src, t < n);
+    }
+    if (p.vec_v) {
+      for (int i = tid; i < CS_C * (CS_CT / 8); i += CS_THREADS) {
+        const int t = i / (CS_CT / 8), c = i % (CS_CT / 8);
+        const bool on = t < n && cta_col + c * 8 < DV;
+        const __nv_bfloat16* src = p.v + ((long long)(tb + (on ? t : 0)) * H + h) * DV + (on ? cta_col + c * 8 : 0);
+        cs_copy16(dst + C::OFF_V + t * C::VPITCH + c * 16, src, on);
+      }
+    } else {
+      for (int i = tid; i < CS_C * CS_CT; i += CS_THREADS) {
+        const int t = i / CS_CT, c = i % CS_CT;
+        const bool on = t < n && cta_col + c < DV;
+        *reinterpret_cast<__nv_bfloat16*>(smem + st * C::STAGE + C::OFF_V + t * C::VPITCH + c * 2) =
+            on ? p.v[((long long)(tb + t) * H + h) * DV + cta_col + c] : __float2bfloat16(0.f);
+      }
+    }
+    const uint8_t* rec = p.rec + ((long long)cs_slot(tb, b) * H + h) * C::REC;
+    for (int i = tid; i < C::REC / 16; i += CS_THREADS) cs_copy16(dst + C::OFF_R + i * 16, rec + i * 16, true);
+  };
+  auto commit = [] { asm volatile("cp.async.commit_group;" ::: "memory"); };
+
+  fetch(t0, 0);
+  commit();
+  if (t0 + CS_C < t1) fetch(t0 + CS_C, 1);
+  commit();
+
+  // S^T in the accumulator layout: S[nt][e] is row 8 nt + 2 quad + (e & 1) of the state, column col + 8 (e >> 1)
+  float S[NT][4];
+  float* pool = p.state ? p.state + ((long long)b * H + h) * DK * DV : nullptr;
+  const long long row_step = MODE == CS_SSD ? 1 : DV, col_step = MODE == CS_SSD ? DK : 1;
+#pragma unroll
+  for (int i = 0; i < NT; ++i)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int c = col + 8 * (e >> 1);
+      S[i][e] = pool && c < DV ? pool[(8 * i + 2 * quad + (e & 1)) * row_step + c * col_step] : 0.f;
+    }
+
+  int st = 0;
+  for (int tb = t0; tb < t1; tb += CS_C) {
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    __syncthreads();                    // this chunk has landed, and every warp has left the stage that is filled next
+    if (tb + 2 * CS_C < t1) fetch(tb + 2 * CS_C, st == 0 ? 2 : st - 1);
+    commit();
+    const uint32_t stage = base + st * C::STAGE;
+    const uint8_t* rec = smem + st * C::STAGE + C::OFF_R;
+    // ---- products with the state: leading parts, and the others
+    float yq[2][2][4], yk[2][2][4];
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) yq[i][j][e] = yk[i][j][e] = 0.f;
+    const uint32_t lrow = (lane & 7) + ((lane >> 4) << 3), lchunk = (lane >> 3) & 1;
+#pragma unroll
+    for (int ks = 0; ks < NK; ++ks) {
+      uint32_t a[3][4], f[4];
+      cs_split_block(S[2 * ks], S[2 * ks + 1], a);
+      if (MODE == CS_DELTA) {
+        cs_ldmatrix(stage + lrow * C::PITCH + (ks * 2 + lchunk) * 16, f);
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          cs_mma(yk[0][j], a[0], f[2 * j], f[2 * j + 1]);
+          cs_mma(yk[1][j], a[1], f[2 * j], f[2 * j + 1]);
+          cs_mma(yk[1][j], a[2], f[2 * j], f[2 * j + 1]);
+        }
+      }
+      cs_ldmatrix(stage + C::OFF_Q + lrow * C::PITCH + (ks * 2 + lchunk) * 16, f);
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        cs_mma(yq[0][j], a[0], f[2 * j], f[2 * j + 1]);
+        cs_mma(yq[1][j], a[1], f[2 * j], f[2 * j + 1]);
+        cs_mma(yq[1][j], a[2], f[2 * j], f[2 * j + 1]);
+      }
+    }
+    // ---- values of this warp's columns, transposed: tokens 8 j + 2 quad + (e & 1), column col + 8 (e >> 1)
+    uint32_t vf[4];
+    cs_ldmatrix_trans(stage + C::OFF_V + lrow * C::VPITCH + (warp * 2 + lchunk) * 16, vf);
+    float r[2][4];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const float2 x = unpack_bf16x2(vf[2 * j]), y = unpack_bf16x2(vf[2 * j + 1]);
+      r[j][0] = x.x; r[j][1] = x.y; r[j][2] = y.x; r[j][3] = y.y;
+    }
+    uint32_t ra[3][4];
+    if (MODE == CS_DELTA) {
+      const float *beta = reinterpret_cast<const float*>(rec + CS_BETA), *eb = reinterpret_cast<const float*>(rec + CS_EB);
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int t = 8 * j + 2 * quad + (e & 1);
+          r[j][e] = beta[t] * r[j][e] - eb[t] * (yk[0][j][e] + yk[1][j][e]);
+        }
+      cs_split_block(r[0], r[1], ra);
+      uint4 tp[3];
+#pragma unroll
+      for (int i = 0; i < 3; ++i) tp[i] = *reinterpret_cast<const uint4*>(rec + CS_T + i * 512 + lane * 16);
+      float lead[2][4], rest[2][4];
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) lead[j][e] = rest[j][e] = 0.f;
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+#define EDL_B(part) (j ? tp[part].z : tp[part].x), (j ? tp[part].w : tp[part].y)
+        cs_mma(rest[j], ra[2], EDL_B(0));
+        cs_mma(rest[j], ra[0], EDL_B(2));
+        cs_mma(rest[j], ra[1], EDL_B(1));
+        cs_mma(rest[j], ra[1], EDL_B(0));
+        cs_mma(rest[j], ra[0], EDL_B(1));
+        cs_mma(lead[j], ra[0], EDL_B(0));
+#pragma unroll
+        for (int e = 0; e < 4; ++e) r[j][e] = lead[j][e] + rest[j][e];
+      }
+      cs_split_block(r[0], r[1], ra);
+    } else {                            // the inputs are exact in one part
+#pragma unroll
+      for (int i = 0; i < 4; ++i) ra[0][i] = vf[i];
+    }
+    // ---- the state behind the chunk
+    {
+      const float* tail = reinterpret_cast<const float*>(rec + CS_TAIL);
+      const float total = *reinterpret_cast<const float*>(rec + CS_TOTAL);
+      float rs[2][4];
+      uint32_t sa[3][4];
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) rs[j][e] = r[j][e] * tail[8 * j + 2 * quad + (e & 1)];
+      cs_split_block(rs[0], rs[1], sa);
+      const uint32_t trow = lane & 15, tchunk = lane >> 4;
+#pragma unroll
+      for (int i = 0; i < NK; ++i) {
+        uint32_t f[4];
+        cs_ldmatrix_trans(stage + trow * C::PITCH + (i * 2 + tchunk) * 16, f);
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          float d[4] = {0.f, 0.f, 0.f, 0.f};
+          cs_mma(d, sa[2], f[2 * j], f[2 * j + 1]);
+          cs_mma(d, sa[1], f[2 * j], f[2 * j + 1]);
+          cs_mma(d, sa[0], f[2 * j], f[2 * j + 1]);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) S[2 * i + j][e] = fmaf(total, S[2 * i + j][e], d[e]);
+        }
+      }
+    }
+    // ---- outputs
+    {
+      const float* es = reinterpret_cast<const float*>(rec + CS_ES);
+      uint4 tp[3];
+#pragma unroll
+      for (int i = 0; i < 3; ++i) tp[i] = *reinterpret_cast<const uint4*>(rec + CS_P + i * 512 + lane * 16);
+      const int n = min(CS_C, t1 - tb);
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        float lead[4] = {0.f, 0.f, 0.f, 0.f}, rest[4] = {0.f, 0.f, 0.f, 0.f};
+        if (MODE == CS_DELTA) {
+          cs_mma(rest, ra[2], EDL_B(0));
+          cs_mma(rest, ra[0], EDL_B(2));
+          cs_mma(rest, ra[1], EDL_B(1));
+          cs_mma(rest, ra[1], EDL_B(0));
+          cs_mma(rest, ra[0], EDL_B(1));
+        } else {
+          cs_mma(rest, ra[0], EDL_B(2));
+          cs_mma(rest, ra[0], EDL_B(1));
+        }
+        cs_mma(lead, ra[0], EDL_B(0));
+#undef EDL_B
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int t = 8 * j + 2 * quad + (e & 1), c = col + 8 * (e >> 1);
+          const float o = es[t] * (yq[0][j][e] + yq[1][j][e]) + (lead[e] + rest[e]);
+          if (t < n && c < DV) p.o[((long long)(tb + t) * H + h) * DV + c] = __float2bfloat16(o);
+        }
+      }
+    }
+    st = st == CS_STAGES - 1 ? 0 : st + 1;
+  }
+  if (pool) {
+#pragma unroll
+    for (int i = 0; i < NT; ++i)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int c = col + 8 * (e >> 1);
+        if (c < DV) pool[(8 * i + 2 * quad + (e & 1)) * row_step + c * col_step] = S[i][e];
+      }
+  }
+}
+
+template <int MODE, int DK>
+int run_chunk_scan(const CsParams& p, cudaStream_t s) {
+  int per = 1;                          // heads that share a chunk's products
+  if (MODE == CS_SSD)
+    while (per < 8 && (p.H / p.G) % (2 * per) == 0) per *= 2;
+  chunk_coef_kernel<MODE, DK><<<dim3(p.T / CS_C + p.B + 1, (p.H / per + 3) / 4), 128, 0, s>>>(p, per);
+  if (check_cuda(cudaGetLastError(), "chunk_coef launch")) return -1;
+  chunk_scan_kernel<MODE, DK><<<dim3((p.DV + CS_CT - 1) / CS_CT, p.H, p.B), CS_THREADS, 0, s>>>(p);
+  return check_cuda(cudaGetLastError(), "chunk_scan launch");
+}
+
+bool cs_aligned(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+
+int cs_check(const char* who, CsParams& p, int DK) {
+  if (p.H < 1 || p.H > 65535 || p.B > 65535 || p.DV < 1 || p.DV > 256 || !p.rec || !cs_aligned(p.rec) || !cs_aligned(p.q) ||
+      !cs_aligned(p.k) || (DK & 15)) {
+    set_last_error("%s: sizes (B=%d, H=%d, DK=%d, DV=%d) or unaligned operands", who, p.B, p.H, DK, p.DV);
+    return -1;
+  }
+  p.vec_v = p.DV % 8 == 0 && cs_aligned(p.v);
+  return 0;
+}
+
+}  // namespace
+}  // namespace edl
+
+using namespace edl;
+
+// q, k [T, H, DK], v [T, H, DV], beta [T, H] or null: bf16; g fp32 [T, H] or null; state fp32 [nseq, H, DK, DV] or null; o bf16
+// [T, H, DV]; rec: workspace of (T / 16 + nseq + 1) * H * 3344 bytes. DK 32, 64 or 128, DV up to 256.
+EDL_HOST_API int edl_delta_rule_chunks(const void* q, const void* k, const void* v, const float* g, const void* beta,
+                                       const int* cu, int T, int nseq, int H, int DK, int DV, float scale, float* state, void* o,
+                                       void* rec, void* stream) {
+  if (nseq <= 0 || H <= 0 || T <= 0) return 0;
+  CsParams p{};
+  p.q = (const __nv_bfloat16*)q; p.k = (const __nv_bfloat16*)k; p.v = (const __nv_bfloat16*)v; p.g = g;
+  p.beta = (const __nv_bfloat16*)beta; p.cu = cu; p.T = T; p.B = nseq; p.H = p.G = H; p.DV = DV; p.scale = scale;
+  p.rec = (uint8_t*)rec; p.state = state; p.o = (__nv_bfloat16*)o;
+  if (cs_check("edl_delta_rule_chunks", p, DK)) return -1;
+  cudaStream_t s = (cudaStream_t)stream;
+  switch (DK) {
+    case 32: return run_chunk_scan<CS_DELTA, 32>(p, s);
+    case 64: return run_chunk_scan<CS_DELTA, 64>(p, s);
+    case 128: return run_chunk_scan<CS_DELTA, 128>(p, s);
+  }
+  set_last_error("edl_delta_rule_chunks: key head_dim %d not in {32, 64, 128}", DK);
+  return -1;
+}
+
+// x [T, H, P], dt [T, H], B, C [T, G, N]: bf16; A, D, dt_bias fp32 [H] (D, dt_bias or null); state fp32 [nseq, H, P, N] or
+// null; y bf16 [T, H, P]; rec: workspace of (T / 16 + nseq + 1) * H * 1680 bytes. N 16, 32, 64 or 128, P up to 256.
+EDL_HOST_API int edl_ssd_scan_chunks(const void* x, const void* dt, const float* A, const void* B, const void* C,
+                                     const float* D, const float* dt_bias, int softplus, const int* cu, int T, int nseq, int H,
+                                     int P, int G, int N, float* state, void* y, void* rec, void* stream) {
+  if (nseq <= 0 || H <= 0 || T <= 0) return 0;
+  if (G < 1 || H % G) {
+    set_last_error("edl_ssd_scan_chunks: heads %d not a multiple of groups %d", H, G);
+    return -1;
+  }
+  CsParams p{};
+  p.q = (const __nv_bfloat16*)C; p.k = (const __nv_bfloat16*)B; p.v = (const __nv_bfloat16*)x; p.dt = (const __nv_bfloat16*)dt;
+  p.A = A; p.Dskip = D; p.dt_bias = dt_bias; p.softplus = softplus; p.cu = cu; p.T = T; p.B = nseq; p.H = H; p.G = G; p.DV = P;
+  p.scale = 1.f; p.rec = (uint8_t*)rec; p.state = state; p.o = (__nv_bfloat16*)y;
+  if (cs_check("edl_ssd_scan_chunks", p, N)) return -1;
+  cudaStream_t s = (cudaStream_t)stream;
+  switch (N) {
+    case 16: return run_chunk_scan<CS_SSD, 16>(p, s);
+    case 32: return run_chunk_scan<CS_SSD, 32>(p, s);
+    case 64: return run_chunk_scan<CS_SSD, 64>(p, s);
+    case 128: return run_chunk_scan<CS_SSD, 128>(p, s);
+  }
+  set_last_error("edl_ssd_scan_chunks: state size %d not in {16, 32, 64, 128}", N);
+  return -1;
+}

@@ -20,8 +20,9 @@ vp, i32, f32 = _lib.vp, _lib.i32, _lib.f32
 _lib.register("edl_selective_scan", i32, [vp, vp, vp, vp, vp, vp, vp, vp, i32, vp, i32, i32, i32, vp, vp, vp])
 _lib.register("edl_ssd_scan", i32, [vp, vp, vp, vp, vp, vp, vp, i32, vp, i32, i32, i32, i32, i32, vp, vp, vp])
 _lib.register("edl_delta_rule", i32, [vp, vp, vp, vp, vp, i32, vp, i32, i32, i32, i32, f32, vp, vp, vp])
-_lib.register("edl_delta_rule_blocks", i32, [vp, vp, vp, vp, vp, i32, vp, i32, i32, i32, i32, i32, f32, vp, vp, vp, vp])
-_lib.register("edl_ssd_scan_blocks", i32, [vp, vp, vp, vp, vp, vp, vp, i32, vp, i32, i32, i32, i32, i32, i32, vp, vp, vp, vp])
+_lib.register("edl_delta_rule_blocks", i32, [vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, f32, vp, vp, vp, vp])
+_lib.register("edl_delta_rule_chunks", i32, [vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, f32, vp, vp, vp, vp])
+_lib.register("edl_ssd_scan_chunks", i32, [vp, vp, vp, vp, vp, vp, vp, i32, vp, i32, i32, i32, i32, i32, i32, vp, vp, vp, vp])
 _lib.register("edl_ragged_conv1d", i32, [vp, vp, vp, vp, vp, i32, i32, i32, i32, vp, vp, vp])
 _lib.register("edl_hgrn2_scan", i32, [vp, i32, _lib.i64, vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, vp, vp, vp])
 _lib.register("edl_hgrn2_decode", i32, [vp, i32, _lib.i64, vp, vp, vp, vp, vp, vp, f32, vp, i32, i32, i32, i32, vp])
@@ -46,14 +47,21 @@ def _use_kernel(*ts) -> bool:
         x is not None and x.requires_grad for x in ts))
 
 
-def _block_records(total: int, nseq: int, heads: int, *rows: torch.Tensor) -> torch.Tensor | None:
-    """Workspace of the scans that take eight tokens at a time (``csrc/block_scan.cu``), or None where the one-token kernels
-    run: steps of mostly single tokens, because a block costs the same for one token as for eight (delta rule, 64 sequences,
-    16 heads of 128 x 128: 1 token 84 against 50 us, 2 tokens 80 against 73, 4 tokens 83 against 117, 8 tokens 85 against
-    203), and rows that do not start on 16 bytes."""
-    if total < 4 * nseq or any(t.data_ptr() % 16 for t in rows):
+def _scan_records(total: int, nseq: int, heads: int, chunk: int, size: int, *rows: torch.Tensor) -> torch.Tensor | None:
+    """Workspace (``size`` bytes per chunk and head) of the scans that take ``chunk`` tokens at a time (``csrc/chunk_scan.cu``
+    sixteen, ``csrc/block_scan.cu`` eight), or None where the one-token kernels run: rows that do not start on 16 bytes, and
+    steps of mostly single tokens. For the chunks these are the small ones only, where a second launch costs more than it
+    saves: 16 heads of 128 x 128, chunks against tokens, 64 sequences of 1, 2, 4, 8 tokens 48, 50, 52, 52 us against 51, 74,
+    118, 212 (state space of 64 x 128: 38, 38, 38, 40 against 81, 83, 87, 98); one sequence of 4 or 16 tokens 34, 34 us against
+    24, 54. A block on the FMA pipe costs the same for one token as for eight: with a decay per channel, blocks against
+    tokens, the same steps 88, 89, 81, 85 us against 58, 88, 148, 274."""
+    if chunk == 16:
+        few = total < 8 * nseq and nseq * heads < 1024
+    else:
+        few = total < 4 * nseq
+    if few or any(t.data_ptr() % 16 for t in rows):
         return None
-    return torch.empty((total // 8 + nseq + 1) * heads * 100, dtype=torch.float32, device=rows[0].device)
+    return torch.empty((total // chunk + nseq + 1) * heads * size, dtype=torch.uint8, device=rows[0].device)
 
 
 # ----------------------------------------------------------------------------------------- Mamba-1
@@ -264,11 +272,11 @@ def ssd_scan(x, dt, A, B, C, D=None, dt_bias=None, softplus=True, cu_seqlens=Non
         x, dt, A, B, C = x.contiguous(), dt.contiguous(), A.float().contiguous(), B.contiguous(), C.contiguous()
         D = None if D is None else D.float().contiguous()
         dt_bias = None if dt_bias is None else dt_bias.float().contiguous()
-        rec = _block_records(total, nseq, H, B, C)
+        rec = _scan_records(total, nseq, H, 16, 1680, B, C)
         args = (x.data_ptr(), dt.data_ptr(), A.data_ptr(), B.data_ptr(), C.data_ptr(), _lib.ptr(D), _lib.ptr(dt_bias),
                 int(softplus), cu.data_ptr())
         if rec is not None:
-            _lib.call("edl_ssd_scan_blocks", *args, total, nseq, H, P, G, N, _lib.ptr(state), y.data_ptr(), rec.data_ptr(),
+            _lib.call("edl_ssd_scan_chunks", *args, total, nseq, H, P, G, N, _lib.ptr(state), y.data_ptr(), rec.data_ptr(),
                       _lib.stream_ptr())
         else:
             _lib.call("edl_ssd_scan", *args, nseq, H, P, G, N, _lib.ptr(state), y.data_ptr(), _lib.stream_ptr())
@@ -364,13 +372,14 @@ def gated_delta_rule(q, k, v, g=None, beta=None, scale=None, cu_seqlens=None, st
         g = None if g is None else g.float().contiguous()
         beta = None if beta is None else beta.to(torch.bfloat16).contiguous()
         scale = float(scale if scale is not None else DK ** -0.5)
-        rec = _block_records(total, nseq, H, q, k, *([g] if per_channel else []))
-        args = (q.data_ptr(), k.data_ptr(), v.data_ptr(), _lib.ptr(g), _lib.ptr(beta), per_channel, cu.data_ptr())
+        args = (q.data_ptr(), k.data_ptr(), v.data_ptr(), _lib.ptr(g), _lib.ptr(beta))
+        rec = _scan_records(total, nseq, H, 8, 288, q, k, g) if per_channel else _scan_records(total, nseq, H, 16, 3344, q, k)
         if rec is not None:
-            _lib.call("edl_delta_rule_blocks", *args, total, nseq, H, DK, DV, scale, _lib.ptr(state), o.data_ptr(),
-                      rec.data_ptr(), _lib.stream_ptr())
+            _lib.call("edl_delta_rule_blocks" if per_channel else "edl_delta_rule_chunks", *args, cu.data_ptr(), total, nseq, H, DK,
+                      DV, scale, _lib.ptr(state), o.data_ptr(), rec.data_ptr(), _lib.stream_ptr())
         else:
-            _lib.call("edl_delta_rule", *args, nseq, H, DK, DV, scale, _lib.ptr(state), o.data_ptr(), _lib.stream_ptr())
+            _lib.call("edl_delta_rule", *args, per_channel, cu.data_ptr(), nseq, H, DK, DV, scale, _lib.ptr(state), o.data_ptr(),
+                      _lib.stream_ptr())
         return o
     if (g is None or g.dim() == 2) and q.shape[0] > 16:
         return delta_rule_chunked(q, k, v, g, beta, scale, cu_seqlens, state)
