@@ -61,6 +61,26 @@ def _splitk_plan(M: int, N: int, K: int, device) -> int:
     return best
 
 
+def _skinny_plan(M: int, N: int, K: int, device) -> int:
+    """CTAs that share the reduction of a 128-column tile in the weight-streaming kernel (0 = use the other kernels).
+
+    Up to 1.6 CTAs per SM: with more, clusters of this size no longer all fit at once and the last ones run alone. One
+    B200, weights from HBM, us (N x K; the other kernels against 1, 2, 4, 6, 8 CTAs per tile):
+      1 row:    6144 x 4096   19.0 / 19.0 13.8 14.0 16.9 15.7     28672 x 4096  66.2 / 41.4 41.8 49.8 50.7 54.3
+                4096 x 14336  32.8 / 54.3 32.4 24.7 24.0 23.2      4096 x 4096  16.4 / 18.4 12.6 10.6 10.2 10.2
+      48 rows:  6144 x 4096   18.9 / 24.3 16.9 15.0 19.7 18.7     28672 x 4096  47.6 / 44.7 47.0 55.2 58.6 63.1
+                4096 x 14336  30.4 / 68.8 40.1 27.7 26.6 25.8      4096 x 4096  14.9 / 23.4 15.3 12.1 11.9 11.9
+      128 rows: 6144 x 4096   20.8 / 31.9 21.2 18.7 24.8 25.2     28672 x 4096  49.3 / 50.3 56.6 68.7 74.3 86.3
+    Matrices whose tiles fill the GPU on their own gain up to 64 rows (45.8 against 48.2 us); above that a CTA loads as
+    many activations as weights and the kernel with two accumulators is as fast or faster.
+    """
+    if M > 128:
+        return 0
+    most = min(8, 8 * sm_count(device) // (5 * ((N + 127) // 128)), (K + 63) // 64 // 2)
+    cluster = max(c for c in (1, 2, 4, 6, 8) if c <= max(1, most))
+    return 0 if M > 64 and cluster == 1 else cluster
+
+
 def _pair_splitk_plan(M: int, N: int, K: int, device) -> int:
     """K slices for the CTA-pair split-K kernel (0 = use the other kernels).
 
@@ -156,6 +176,12 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
     lda = a.stride(0) if a.shape[0] > 1 else a.shape[1]
     ldb = b.stride(0) if b.shape[0] > 1 else b.shape[1]
     ldc = out.stride(0) if out.shape[0] > 1 else out.shape[1]
+    if not (a_mn or b_mn or max_ctas or force_bn or pair_splits) and (out.dtype == torch.float32 or not accumulate):
+        cluster = _skinny_plan(M, N, K, a.device)
+        if cluster and out.data_ptr() % 16 == 0 and ldc % (4 if out.dtype == torch.float32 else 8) == 0:
+            _lib.call("edl_gemm_skinny", a.data_ptr(), b.data_ptr(), out.data_ptr(), _lib.ptr(bias), M, N, K, lda, ldb, ldc,
+                      cluster, flags, _lib.status_word(a.device).data_ptr(), _lib.stream_ptr())
+            return out
     if not (a_mn or b_mn or accumulate or max_ctas) and out.dtype == torch.bfloat16 and force_bn in (0, 512):
         ps = pair_splits or (_pair_splitk_plan(M, N, K, a.device) if not force_bn else 0)
         if ps > 1 or (ps == 1 and pair_splits):

@@ -148,6 +148,35 @@ def test_gemm_skinny_uses_split_k(M, N, K):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("M,N,K", [(1, 128, 64), (3, 200, 136), (16, 1000, 512), (17, 31, 4096), (64, 520, 1000),
+                                   (128, 300, 2048)])
+@pytest.mark.parametrize("cluster", [1, 2, 3, 8])
+def test_gemm_weight_streaming(M, N, K, cluster, monkeypatch):
+    """The kernel for a few rows at the edges of its tiles (rows around 16, columns around 128, ragged reductions), every
+    way of cutting the reduction: bf16 with bias, and fp32 added to what is there."""
+    from easydel_b200.ops import kernels as K_
+
+    cluster = min(cluster, (K + 63) // 64)
+    monkeypatch.setattr(K_, "_skinny_plan", lambda *a: cluster)
+    torch.manual_seed(M + N + K)
+    a = torch.randn(M, K, device="cuda", dtype=torch.bfloat16)
+    w = torch.randn(N, K, device="cuda", dtype=torch.bfloat16)
+    bias = torch.randn(N, device="cuda", dtype=torch.bfloat16)
+    ref = a.double() @ w.double().t()
+    pitch = (N + 7) // 8 * 8
+    out = torch.full((M, pitch), 7.0, device="cuda", dtype=torch.bfloat16)
+    K_.gemm(a, w, out=out[:, :N], bias=bias)
+    # products are exact in fp32; the sum of K of them, each about 1, is off by less than K * 2^-23 of its largest partial
+    # sum, and bf16 rounds the result by 2^-9
+    tol = 2.0 ** -23 * K * 4 * K ** 0.5
+    assert ((out[:, :N].double() - ref - bias.double()).abs() <= 2.0 ** -8 * (ref + bias.double()).abs() + tol).all()
+    assert (out[:, N:] == 7.0).all()
+    acc = torch.ones(M, pitch, device="cuda")
+    K_.gemm(a, w, out=acc[:, :N], accumulate=True)
+    assert ((acc[:, :N].double() - 1 - ref).abs() <= tol).all() and (acc[:, N:] == 1.0).all()
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("M,N,K,splits", [(256, 1280, 8192, 4), (200, 7168, 4096, 2), (64, 520, 1024, 3),
                                           (256, 8192, 1024, 1), (384, 768, 2048, 5)])
 def test_pair_splitk_matches_fp32(M, N, K, splits):
