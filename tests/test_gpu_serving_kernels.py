@@ -209,6 +209,40 @@ def test_latent_decode_attention_kernel(B, H, ctx, splits):
         assert err < 2e-2, (b, float(err))
 
 
+@pytest.mark.parametrize("H,L,R", [(17, 512, 64), (64, 512, 64), (128, 512, 64), (130, 512, 64), (40, 128, 64), (33, 320, 32),
+                                   (20, 72, 24), (18, 504, 72), (24, 256, 0), (5, 512, 64)])
+@pytest.mark.parametrize("lens", [[1], [64, 65, 0, 700, 129], [33] * 20 + [2000], [190] * 90])
+@pytest.mark.parametrize("window,splits", [(0, 1), (100, 1), (0, 3)])
+def test_latent_decode_many_heads(H, L, R, lens, window, splits):
+    """Latent decode attention by either kernel: partial tiles, empty sequences, windows, every cluster size (by the number
+    of sequences), row widths that fill their last box or not, maxima that grow along a sequence, sinks."""
+    from easydel_b200.ops import _lib, serving as S
+
+    torch.manual_seed(H + L)
+    B, W = len(lens), L + R
+    per = 40 if H > 16 else (max(lens) + 127) // 128        # the rule between the kernels goes by the table's width
+    pages = (torch.randn(B * per + 1, 128, 1, W, device="cuda") * 0.5).to(torch.bfloat16)
+    table = (torch.randperm(B * per, device="cuda") + 1).view(B, per).to(torch.int32)
+    q = (torch.randn(B, H, W, device="cuda") * 0.5).to(torch.bfloat16)
+    if lens[-1] > 1000:      # one late row that every head of the last sequence prefers by far
+        pages[table[-1, lens[-1] // 128].long(), lens[-1] % 128 - 1] = q[-1].float().sum(0).to(torch.bfloat16) * 8
+    sinks = torch.randn(H, device="cuda")
+    scale = 0.3 * W ** -0.5 * 8
+    kv = torch.tensor(lens, dtype=torch.int32, device="cuda")
+    q_lat = q[..., :L].transpose(0, 1).contiguous().transpose(0, 1) if H % 2 else q[..., :L]     # both orders of heads
+    o = S.latent_decode(q_lat, q[..., L:], pages, kv, table, scale=scale, window=window, sinks=sinks, num_splits=splits)
+    torch.cuda.synchronize()
+    _lib.check_status()
+    assert o.shape == (B, H, L)
+    for b, n in enumerate(lens):
+        rows = pages[table[b].long()].reshape(-1, W)[max(0, n - window) if window else 0:n].double()
+        s = torch.cat([q[b].double() @ rows.t() * scale, sinks.double()[:, None]], 1)
+        want = torch.softmax(s, -1)[:, :-1] @ rows[:, :L]
+        # probabilities, outputs (and partial outputs of the splits) are rounded to bf16: 2^-9 of the largest row each
+        tol = 3 * 2.0 ** -8 * float(rows.abs().max() if n else 0)
+        assert float((o[b].double() - want).abs().max()) <= tol, (b, n)
+
+
 def _hash_u32(x):
     x &= 0xFFFFFFFF
     x = ((x ^ (x >> 16)) * 0x7FEB352D) & 0xFFFFFFFF
