@@ -25,7 +25,7 @@ from ..ops import _lib
 _lib.register("edl_dequant_bf16", _lib.i32, [_lib.vp, _lib.vp, _lib.vp, _lib.vp, _lib.i32, _lib.i32, _lib.i32, _lib.i32,
                                              _lib.vp, _lib.i64, _lib.vp])
 _lib.register("edl_qgemv", _lib.i32, [_lib.vp, _lib.i64, _lib.vp, _lib.vp, _lib.vp, _lib.vp, _lib.i32, _lib.i32,
-                                      _lib.i32, _lib.i32, _lib.i32, _lib.vp, _lib.i64, _lib.vp, _lib.vp, _lib.vp])
+                                      _lib.i32, _lib.i32, _lib.i32, _lib.vp, _lib.i64, _lib.vp, _lib.vp])
 
 _NF4 = [-1.0, -0.6961928009986877, -0.5250730514526367, -0.39491748809814453, -0.28444138169288635,
         -0.18477343022823334, -0.09105003625154495, 0.0, 0.07958029955625534, 0.16093020141124725,
@@ -192,6 +192,9 @@ def quantize(w: torch.Tensor, config: EasyDeLQuantizationConfig | str = "nf4") -
                            zeros.contiguous() if zeros is not None else None, lut, bits, group, (N, K), cfg.dtype)
 
 
+QGEMV_ROWS = 16      # rows up to which the fused product is the faster one
+
+
 def quantized_matmul(x: torch.Tensor, q: QuantizedTensor, bias: torch.Tensor | None = None) -> torch.Tensor:
     """``x @ W^T`` for a quantised ``W``; picks the fused GEMV for decode-sized inputs."""
     N, K = q.shape
@@ -199,12 +202,13 @@ def quantized_matmul(x: torch.Tensor, q: QuantizedTensor, bias: torch.Tensor | N
     M = x2.shape[0]
     per16 = 32 if q.bits == 4 else 16
     if x2.is_cuda and _lib.available() and x2.dtype == torch.bfloat16:
-        if M <= 8 and q.group % per16 == 0:
-            x32 = x2.float().contiguous()     # the kernel reads fp32 activations (a few rows: converted once)
+        if M <= QGEMV_ROWS and q.group % per16 == 0:
+            if x2.stride(1) != 1 or x2.stride(0) % 8 or x2.data_ptr() % 16:
+                x2 = x2.clone(memory_format=torch.contiguous_format)
             out = torch.empty(M, N, dtype=torch.bfloat16, device=x.device)
-            _lib.call("edl_qgemv", x32.data_ptr(), K, q.codes.data_ptr(),
+            _lib.call("edl_qgemv", x2.data_ptr(), x2.stride(0), q.codes.data_ptr(),
                       q.scales.data_ptr(), _lib.ptr(q.zeros), q.lut.data_ptr(), q.bits, M, N, K, q.group,
-                      out.data_ptr(), N, _lib.ptr(bias), _lib.status_word(x.device).data_ptr(), _lib.stream_ptr())
+                      out.data_ptr(), N, _lib.ptr(bias), _lib.stream_ptr())
             return out.view(*x.shape[:-1], N)
         from ..ops import functional as F
 

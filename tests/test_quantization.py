@@ -45,6 +45,38 @@ def test_quantizer_replaces_linears_and_keeps_outputs_close():
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("fmt,block", [("nf4", 64), ("nf4", 128), ("nf4", 96), ("affine", 32), ("a4bit", 64), ("mxfp4", None),
+                                       ("int8", 128), ("int8", 48), ("a8bit", 32), ("mxfp8", None), ("nvfp8", None)])
+@pytest.mark.parametrize("N,K", [(5, 96), (17, 288), (130, 1152), (1000, 6240)])
+@pytest.mark.parametrize("odd", [False, True])
+def test_fused_product_at_its_edges(fmt, block, N, K, odd):
+    """The fused product of a few rows: ragged weight rows and reductions, groups within, across and beyond a lane's 16 bytes
+    of codes, 1 to 16 activation rows; ``odd``: codes that start on 4 bytes only, strided activations, a bias."""
+    from easydel_b200.layers.quantization import QuantizedTensor
+
+    if block is not None and K % block:
+        K = max(1, K // block) * block
+    torch.manual_seed(N)
+    q = quantize(torch.randn(N, K, device="cuda") * 0.05, EasyDeLQuantizationConfig(fmt, block_size=block))
+    if odd:
+        raw = torch.empty(q.codes.numel() + 4, dtype=torch.uint8, device="cuda")
+        codes = raw[4:].view(q.codes.shape)
+        codes.copy_(q.codes)
+        q = QuantizedTensor(codes, q.scales, q.zeros, q.lut, q.bits, q.group, q.shape, q.fmt)
+    w = dequantize_reference(q).double()
+    bias = torch.randn(N, device="cuda", dtype=torch.bfloat16) if odd else None
+    for M in (1, 3, 8, 9, 16):
+        x = torch.randn(M, K + (3 if odd else 0), device="cuda").to(torch.bfloat16)[:, :K]
+        y = quantized_matmul(x, q, bias)
+        ref = x.double() @ w.t() + (0 if bias is None else bias.double())
+        # bf16 rounds the result by 2^-9; values keep 16 bits (2^-17 each), sums are fp32
+        tol = 2.0 ** -8 * ref.abs() + 2.0 ** -16 * (x.double().abs() @ w.abs().t())
+        assert ((y.double() - ref).abs() <= tol).all(), M
+    if not odd:
+        assert torch.equal(q.dequantize(), dequantize_reference(q).to(torch.bfloat16))
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("fmt", ["int8", "a4bit", "nf4", "mxfp4", "nvfp4", "mxfp8", "nvfp8"])
 @pytest.mark.parametrize("M", [1, 5, 8, 64])
 def test_cuda_kernels_match_reference(fmt, M):
