@@ -704,6 +704,10 @@ class DecoderModel(EasyDeLBaseModule):
             x = tpar.shard_rows(self.sp, x)
         else:
             self.sp.end()
+        if segment_ids is not None and past_key_values is None and segment_ids.is_cuda and segment_ids.dim() == 2:
+            from ...ops.attention import with_segment_plan
+
+            segment_ids = with_segment_plan(segment_ids)
         policy = self.gradient_checkpointing_policy() not in ("", "everything_saveable")
         pending = None
         all_hidden = [] if output_hidden_states else None

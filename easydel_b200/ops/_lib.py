@@ -124,8 +124,16 @@ def use_kernels(*tensors: torch.Tensor) -> bool:
     return True
 
 
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+_device_index = getattr(torch._C, "_cuda_getDevice", None)
+
+
 def stream_ptr() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    """The current stream of the current device. Every launch asks for it: through a ``Stream`` object it took 6 us, a tenth
+    of the host time of a small training step."""
+    if _raw_stream is None or _device_index is None:
+        return torch.cuda.current_stream().cuda_stream
+    return _raw_stream(_device_index())
 
 
 def ptr(t: torch.Tensor | None) -> int | None:
