@@ -4,6 +4,7 @@ from __future__ import annotations
 
 import torch
 from torch import nn
+from torch.nn.modules.module import _global_forward_hooks
 
 from ..ops import functional as F, stream
 from ..ops.reference import ACT2FN
@@ -29,6 +30,12 @@ class GatedMLP(nn.Module):
     # fixed muP multipliers on the gate pre-activation and on the output (Falcon-H1); 1.0 elsewhere
     gate_multiplier: float = 1.0
     down_multiplier: float = 1.0
+
+    def ends_in_product(self) -> bool:
+        """Whether :meth:`forward` returns what ``down_proj`` computes, with nothing in between that could read it."""
+        d = self.down_proj
+        return (type(self) is GatedMLP and type(d) is RowParallelLinear and d.tp_size == 1 and d.scale is None
+                and self.down_multiplier == 1.0 and not (self._forward_hooks or d._forward_hooks or _global_forward_hooks))
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         gu = self.gate_up_proj(x)

@@ -32,7 +32,7 @@ from ...layers.linears import ColumnParallelLinear
 from ...layers.mlp import GatedMLP, PlainMLP
 from ...layers.moe import MoEBlock
 from ...layers.norms import LayerNorm, RMSNorm
-from ...ops import functional as F, stream
+from ...ops import functional as F, remat, stream
 
 
 @dataclass
@@ -513,7 +513,9 @@ class DecoderLayer(nn.Module):
                 h, x = self.input_layernorm.forward_with_residual(pending, x)
             a = self._mix(h, positions, segment_ids, cache_view, attn_meta)
             h, x = self.post_attention_layernorm.forward_with_residual(a, x)
-            m = self.mlp(h)
+            with remat.returned_as_is(type(self).forward is DecoderLayer.forward and not self._forward_hooks
+                                      and type(self.mlp) is GatedMLP and self.mlp.ends_in_product()):
+                m = self.mlp(h)
             if self.is_moe:
                 m, rl = m
             return x, m, rl
@@ -642,10 +644,8 @@ class DecoderModel(EasyDeLBaseModule):
                                         self.remat_policy())
         if policy and self.training and torch.is_grad_enabled() and cache_view is None:
             # recompute unit under the configured save policy (full recompute, saved dots, saved names ...)
-            from ...ops import remat
-
             return remat.recompute_unit(lambda a, b, c, d: layer(a, b, c, d, None, None), self.remat_policy(),
-                                        (x, _resolve(pending), positions, segment_ids))
+                                        (x, _resolve(pending), positions, segment_ids), whole_layer=True)
         return layer(x, pending, positions, segment_ids, cache_view, attn_meta)
 
     def forward(self, input_ids: torch.Tensor | None = None, attention_mask: torch.Tensor | None = None,

@@ -31,7 +31,8 @@ class _LinearFn(torch.autograd.Function):
         hit, y = remat.saved_output(name, "dot")   # recompute of a unit that kept this product: no GEMM
         if not hit:
             y = torch.empty((*x.shape[:-1], w.shape[0]), dtype=x.dtype, device=x.device)
-            K.gemm(x2, w, bias=bias, out=y.view(-1, w.shape[0]))
+            if not remat.unread_output(name):
+                K.gemm(x2, w, bias=bias, out=y.view(-1, w.shape[0]))
             remat.keep_output(name, "dot", y)
         ctx.save_for_backward(x2, w)
         ctx.has_bias = bias is not None

@@ -140,3 +140,41 @@ def test_activation_save_policies_match_no_checkpointing(policy, targets):
     if policy != "nothing_saveable":
         _, _, n_full = run("nothing_saveable", None)
         assert n1 < n_full, (n1, n_full)
+
+
+@pytest.mark.parametrize("span", ["layer", "two layers", "layer and a hook"])
+def test_recompute_leaves_out_only_what_nobody_reads(span):
+    """Gradients through recomputed layers equal those of layers that keep their activations, bit for bit: a unit that is one
+    layer (whose last product need not run again), a unit of two (whose first layer's is read), a layer with a hook on it."""
+    from easydel_b200.modules.llama import LlamaConfig, LlamaForCausalLM
+    from easydel_b200.ops import remat
+
+    cfg = LlamaConfig(vocab_size=256, hidden_size=256, intermediate_size=512, num_hidden_layers=2, num_attention_heads=4,
+                      num_key_value_heads=2, head_dim=64, max_position_embeddings=256)
+    model = LlamaForCausalLM.sequential_init(cfg, dtype=torch.bfloat16, param_dtype=torch.bfloat16, device="cuda", seed=3).train()
+    a, b = model.model.layers
+    if span == "layer and a hook":
+        a.mlp.down_proj.register_forward_hook(lambda m, i, o: o * 2)
+    pos = torch.arange(200, device="cuda")[None]
+    x0 = torch.randn(1, 200, 256, device="cuda", dtype=torch.bfloat16)
+
+    def pair(x):
+        y, p, _ = a(x, None, pos, None, None, None)
+        return b(y, p, pos, None, None, None)[:2]
+
+    def units(x):
+        policy = remat.get_policy("nothing_saveable")
+        if span == "two layers":
+            return remat.recompute_unit(pair, policy, (x,))
+        y, p, _ = remat.recompute_unit(lambda t: a(t, None, pos, None, None, None), policy, (x,), whole_layer=True)
+        return remat.recompute_unit(lambda t, u: b(t, u, pos, None, None, None), policy, (y, p), whole_layer=True)[:2]
+
+    got = []
+    for f in (pair, units):
+        model.zero_grad(set_to_none=True)
+        x = x0.clone().requires_grad_()
+        y, p = f(x)
+        (y.float().square().sum() + p.float().square().sum()).backward()
+        got.append([y.detach(), p.detach(), x.grad] + [w.grad for w in list(a.parameters()) + list(b.parameters())])
+    for u, v in zip(*got):
+        assert torch.equal(u, v)
