@@ -27,8 +27,9 @@
 //
 // 5328 + 2864 tokens, 32 heads of 128 x 128: 0.73 ms (eight tokens at a time on the FMA pipe 1.90 ms, one at a time 19.4 ms);
 // 6000 tokens in three sequences, 64 state-space heads of 64 x 128: 0.32 ms (0.74 ms, 4.4 ms). Bytes at the copy rate: 43 and
-// 18 us. A value that is not finite spoils its column for the whole chunk (a zero weight times infinity), not only from its
-// token on.
+// 18 us. State-space sequences are cut into segments where that fills the GPU (cs_span): 8192 tokens of one sequence, 64 heads
+// 0.93 -> 0.38 ms, 8 heads 0.91 -> 0.09 ms. A value that is not finite spoils its column for the whole chunk (a zero weight
+// times infinity), not only from its token on.
 // Compiled without fast-math.
 #include "common.cuh"
 
@@ -64,7 +65,39 @@ struct CsParams {
   float* state;                      // delta [B, H, DK, DV], state space [B, H, DV, DK]; or null
   __nv_bfloat16* o;                  // [T, H, DV]
   bool vec_v;                        // values can be fetched 16 bytes at a time
+  int seg;                           // tokens of a segment (a multiple of 16), or 0: sequences are walked from end to end
+  float *seg_state, *seg_decay;      // [segments, H, DV, DK], [segments, H]
 };
+
+// Segments of long state-space sequences run side by side: the state behind one is its decay times the state in front of it
+// plus what its tokens leave in an empty state. A first pass computes the latter (48 of the 102 products of a chunk), one
+// thread per element carries states from segment to segment, then every segment runs in full from the state in front of it.
+// A segment's place, as a chunk's: unique and increasing, below T / seg + B + 1.
+struct CsSpan {
+  int b, t0, t1, slot;
+};
+__device__ __forceinline__ CsSpan cs_span(const CsParams& p, int z) {
+  CsSpan s;
+  s.slot = z;
+  if (p.seg == 0) {
+    s.b = z;
+    s.t0 = p.cu[z];
+    s.t1 = p.cu[z + 1];
+    return s;
+  }
+  int lo = 0, hi = p.B;
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (p.cu[mid] / p.seg + mid <= z) lo = mid;
+    else hi = mid;
+  }
+  s.b = lo;
+  const long long first = p.cu[lo], at = first + (long long)(z - ((int)first / p.seg + lo)) * p.seg;
+  const int end = p.cu[lo + 1];
+  s.t0 = at < first || at >= end ? end : (int)at;
+  s.t1 = min(end, (int)min((long long)end, s.t0 + (long long)p.seg));
+  return s;
+}
 
 // A chunk's place in the record array: unique and increasing over (sequence, chunk), below T / 16 + B + 1.
 __device__ __forceinline__ int cs_slot(int t, int b) { return t / CS_C + b; }
@@ -265,15 +298,16 @@ struct CsCfg {
   static_assert(STAGE % 16 == 0 && CS_STAGES * STAGE <= 48 * 1024, "");
 };
 
-template <int MODE, int DK>
+// LOCAL: only the state that a segment's tokens leave in an empty one, and its decay.
+template <int MODE, int DK, bool LOCAL>
 __global__ void __launch_bounds__(CS_THREADS) chunk_scan_kernel(const CsParams p) {
   using C = CsCfg<MODE, DK>;
   constexpr int NT = DK / 8, NK = DK / 16;
   __shared__ __align__(128) uint8_t smem[CS_STAGES * C::STAGE];
   const uint32_t base = smem_u32(smem);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, row = lane >> 2, quad = lane & 3;
-  const int h = blockIdx.y, b = blockIdx.z;
-  const int t0 = p.cu[b], t1 = p.cu[b + 1];
+  const CsSpan span = cs_span(p, blockIdx.z);
+  const int h = blockIdx.y, b = span.b, t0 = span.t0, t1 = span.t1;
   if (t0 >= t1) return;
   const int H = p.H, DV = p.DV, rows = h / (p.H / p.G);
   const int cta_col = blockIdx.x * CS_CT, col = cta_col + warp * 16 + row;    // this lane's columns: col, col + 8
@@ -281,7 +315,7 @@ __global__ void __launch_bounds__(CS_THREADS) chunk_scan_kernel(const CsParams p
   auto fetch = [&](int tb, int st) {
     const int n = min(CS_C, t1 - tb);
     const uint32_t dst = base + st * C::STAGE;
-    for (int i = tid; i < 2 * CS_C * (DK / 8); i += CS_THREADS) {
+    for (int i = tid; i < (LOCAL ? 1 : 2) * CS_C * (DK / 8); i += CS_THREADS) {
       const int which = i / (CS_C * (DK / 8)), t = (i / (DK / 8)) % CS_C, c = i % (DK / 8);
       const __nv_bfloat16* src = (which ? p.q : p.k) + ((long long)(tb + (t < n ? t : 0)) * p.G + rows) * DK + c * 8;
       cs_copy16(dst + which * C::OFF_Q + t * C::PITCH + c * 16, src, t < n);
@@ -313,14 +347,16 @@ __global__ void __launch_bounds__(CS_THREADS) chunk_scan_kernel(const CsParams p
 
   // S^T in the accumulator layout: S[nt][e] is row 8 nt + 2 quad + (e & 1) of the state, column col + 8 (e >> 1)
   float S[NT][4];
-  float* pool = p.state ? p.state + ((long long)b * H + h) * DK * DV : nullptr;
+  float* pool = p.seg ? p.seg_state + ((long long)span.slot * H + h) * DK * DV
+                      : (p.state ? p.state + ((long long)b * H + h) * DK * DV : nullptr);
+  float decay = 1.f;
   const long long row_step = MODE == CS_SSD ? 1 : DV, col_step = MODE == CS_SSD ? DK : 1;
 #pragma unroll
   for (int i = 0; i < NT; ++i)
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       const int c = col + 8 * (e >> 1);
-      S[i][e] = pool && c < DV ? pool[(8 * i + 2 * quad + (e & 1)) * row_step + c * col_step] : 0.f;
+      S[i][e] = !LOCAL && pool && c < DV ? pool[(8 * i + 2 * quad + (e & 1)) * row_step + c * col_step] : 0.f;
     }
 
   int st = 0;
@@ -341,7 +377,7 @@ __global__ void __launch_bounds__(CS_THREADS) chunk_scan_kernel(const CsParams p
         for (int e = 0; e < 4; ++e) yq[i][j][e] = yk[i][j][e] = 0.f;
     const uint32_t lrow = (lane & 7) + ((lane >> 4) << 3), lchunk = (lane >> 3) & 1;
 #pragma unroll
-    for (int ks = 0; ks < NK; ++ks) {
+    for (int ks = 0; ks < (LOCAL ? 0 : NK); ++ks) {
       uint32_t a[3][4], f[4];
       cs_split_block(S[2 * ks], S[2 * ks + 1], a);
       if (MODE == CS_DELTA) {
@@ -410,6 +446,7 @@ __global__ void __launch_bounds__(CS_THREADS) chunk_scan_kernel(const CsParams p
     {
       const float* tail = reinterpret_cast<const float*>(rec + CS_TAIL);
       const float total = *reinterpret_cast<const float*>(rec + CS_TOTAL);
+      if (LOCAL) decay *= total;
       float rs[2][4];
       uint32_t sa[3][4];
 #pragma unroll
@@ -434,7 +471,7 @@ __global__ void __launch_bounds__(CS_THREADS) chunk_scan_kernel(const CsParams p
       }
     }
     // ---- outputs
-    {
+    if constexpr (!LOCAL) {
       const float* es = reinterpret_cast<const float*>(rec + CS_ES);
       uint4 tp[3];
 #pragma unroll
@@ -465,7 +502,8 @@ __global__ void __launch_bounds__(CS_THREADS) chunk_scan_kernel(const CsParams p
     }
     st = st == CS_STAGES - 1 ? 0 : st + 1;
   }
-  if (pool) {
+  if (LOCAL && blockIdx.x == 0 && tid == 0) p.seg_decay[(long long)span.slot * H + h] = decay;
+  if (pool && (LOCAL || p.seg == 0)) {
 #pragma unroll
     for (int i = 0; i < NT; ++i)
 #pragma unroll
@@ -476,6 +514,27 @@ __global__ void __launch_bounds__(CS_THREADS) chunk_scan_kernel(const CsParams p
   }
 }
 
+// Turns what the segments of a sequence leave behind into the states in front of them; the state behind the last one goes out.
+__global__ void chunk_carry_kernel(const CsParams p, int n4) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x, h = blockIdx.y, b = blockIdx.z;
+  if (i >= n4) return;
+  const int first = p.cu[b], n = (p.cu[b + 1] - first + p.seg - 1) / p.seg, slot = first / p.seg + b;
+  if (n <= 0) return;
+  float4* pool = p.state ? reinterpret_cast<float4*>(p.state) + ((long long)b * p.H + h) * n4 + i : nullptr;
+  float4* at = reinterpret_cast<float4*>(p.seg_state) + ((long long)slot * p.H + h) * n4 + i;
+  const float* decay = p.seg_decay + (long long)slot * p.H + h;
+  const long long step = (long long)p.H * n4;
+  float4 s = pool ? *pool : make_float4(0.f, 0.f, 0.f, 0.f), next = at[0];
+  for (int k = 0; k < n; ++k) {
+    const float4 left = next;
+    if (k + 1 < n) next = at[(k + 1) * step];
+    const float d = decay[(long long)k * p.H];
+    at[k * step] = s;
+    s = make_float4(fmaf(d, s.x, left.x), fmaf(d, s.y, left.y), fmaf(d, s.z, left.z), fmaf(d, s.w, left.w));
+  }
+  if (pool) *pool = s;
+}
+
 template <int MODE, int DK>
 int run_chunk_scan(const CsParams& p, cudaStream_t s) {
   int per = 1;                          // heads that share a chunk's products
@@ -483,7 +542,17 @@ int run_chunk_scan(const CsParams& p, cudaStream_t s) {
     while (per < 8 && (p.H / p.G) % (2 * per) == 0) per *= 2;
   chunk_coef_kernel<MODE, DK><<<dim3(p.T / CS_C + p.B + 1, (p.H / per + 3) / 4), 128, 0, s>>>(p, per);
   if (check_cuda(cudaGetLastError(), "chunk_coef launch")) return -1;
-  chunk_scan_kernel<MODE, DK><<<dim3((p.DV + CS_CT - 1) / CS_CT, p.H, p.B), CS_THREADS, 0, s>>>(p);
+  const int tiles = (p.DV + CS_CT - 1) / CS_CT, spans = p.seg ? p.T / p.seg + p.B + 1 : p.B;
+  if constexpr (MODE == CS_SSD) {
+    if (p.seg) {
+      chunk_scan_kernel<MODE, DK, true><<<dim3(tiles, p.H, spans), CS_THREADS, 0, s>>>(p);
+      if (check_cuda(cudaGetLastError(), "chunk_scan (segments) launch")) return -1;
+      const int n4 = p.DV * DK / 4;
+      chunk_carry_kernel<<<dim3((n4 + 255) / 256, p.H, p.B), 256, 0, s>>>(p, n4);
+      if (check_cuda(cudaGetLastError(), "chunk_carry launch")) return -1;
+    }
+  }
+  chunk_scan_kernel<MODE, DK, false><<<dim3(tiles, p.H, spans), CS_THREADS, 0, s>>>(p);
   return check_cuda(cudaGetLastError(), "chunk_scan launch");
 }
 
@@ -527,10 +596,17 @@ EDL_HOST_API int edl_delta_rule_chunks(const void* q, const void* k, const void*
 
 // x [T, H, P], dt [T, H], B, C [T, G, N]: bf16; A, D, dt_bias fp32 [H] (D, dt_bias or null); state fp32 [nseq, H, P, N] or
 // null; y bf16 [T, H, P]; rec: workspace of (T / 16 + nseq + 1) * H * 1680 bytes. N 16, 32, 64 or 128, P up to 256.
+// seg: tokens of a segment (a multiple of 16) or 0; segments: workspace of (T / seg + nseq + 1) * H * (P * N + 1) floats,
+// 16-byte aligned, as `state` has to be then.
 EDL_HOST_API int edl_ssd_scan_chunks(const void* x, const void* dt, const float* A, const void* B, const void* C,
                                      const float* D, const float* dt_bias, int softplus, const int* cu, int T, int nseq, int H,
-                                     int P, int G, int N, float* state, void* y, void* rec, void* stream) {
+                                     int P, int G, int N, float* state, void* y, void* rec, int seg, float* segments,
+                                     void* stream) {
   if (nseq <= 0 || H <= 0 || T <= 0) return 0;
+  if (seg < 0 || seg % CS_C || (seg && (!segments || !cs_aligned(segments) || !cs_aligned(state) || T / seg + nseq + 1 > 65535))) {
+    set_last_error("edl_ssd_scan_chunks: segments of %d tokens", seg);
+    return -1;
+  }
   if (G < 1 || H % G) {
     set_last_error("edl_ssd_scan_chunks: heads %d not a multiple of groups %d", H, G);
     return -1;
@@ -539,6 +615,9 @@ EDL_HOST_API int edl_ssd_scan_chunks(const void* x, const void* dt, const float*
   p.q = (const __nv_bfloat16*)C; p.k = (const __nv_bfloat16*)B; p.v = (const __nv_bfloat16*)x; p.dt = (const __nv_bfloat16*)dt;
   p.A = A; p.Dskip = D; p.dt_bias = dt_bias; p.softplus = softplus; p.cu = cu; p.T = T; p.B = nseq; p.H = H; p.G = G; p.DV = P;
   p.scale = 1.f; p.rec = (uint8_t*)rec; p.state = state; p.o = (__nv_bfloat16*)y;
+  p.seg = seg;
+  p.seg_state = segments;
+  if (seg) p.seg_decay = segments + (long long)(T / seg + nseq + 1) * H * P * N;
   if (cs_check("edl_ssd_scan_chunks", p, N)) return -1;
   cudaStream_t s = (cudaStream_t)stream;
   switch (N) {

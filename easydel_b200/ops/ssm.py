@@ -22,7 +22,7 @@ _lib.register("edl_ssd_scan", i32, [vp, vp, vp, vp, vp, vp, vp, i32, vp, i32, i3
 _lib.register("edl_delta_rule", i32, [vp, vp, vp, vp, vp, i32, vp, i32, i32, i32, i32, f32, vp, vp, vp])
 _lib.register("edl_delta_rule_blocks", i32, [vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, f32, vp, vp, vp, vp])
 _lib.register("edl_delta_rule_chunks", i32, [vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, f32, vp, vp, vp, vp])
-_lib.register("edl_ssd_scan_chunks", i32, [vp, vp, vp, vp, vp, vp, vp, i32, vp, i32, i32, i32, i32, i32, i32, vp, vp, vp, vp])
+_lib.register("edl_ssd_scan_chunks", i32, [vp, vp, vp, vp, vp, vp, vp, i32, vp, i32, i32, i32, i32, i32, i32, vp, vp, vp, i32, vp, vp])
 _lib.register("edl_ragged_conv1d", i32, [vp, vp, vp, vp, vp, i32, i32, i32, i32, vp, vp, vp])
 _lib.register("edl_hgrn2_scan", i32, [vp, i32, _lib.i64, vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, vp, vp, vp])
 _lib.register("edl_hgrn2_decode", i32, [vp, i32, _lib.i64, vp, vp, vp, vp, vp, vp, f32, vp, i32, i32, i32, i32, vp])
@@ -62,6 +62,21 @@ def _scan_records(total: int, nseq: int, heads: int, chunk: int, size: int, *row
     if few or any(t.data_ptr() % 16 for t in rows):
         return None
     return torch.empty((total // chunk + nseq + 1) * heads * size, dtype=torch.uint8, device=rows[0].device)
+
+
+def _scan_segment(total: int, nseq: int, units: int, size: int) -> int:
+    """Tokens of a segment of the state-space scan (``csrc/chunk_scan.cu``), 0 to walk sequences from end to end. ``units``: heads
+    times tiles of 64 columns; ``size``: of the state. Segments take half as many products again, which the tensor pipe has to
+    have room for: walked, a sequence of 16-token chunks takes 1.8 us a chunk and all units together 0.0101 us a chunk; cut, a
+    chunk costs 2.6 us of a segment's time and 0.0118 us of the pipe's (states of 128 wide; in proportion for narrower ones).
+    One B200, walked / cut, us: 8192 tokens of 64 heads 933 / 382, of 8 heads 913 / 92; three sequences of 6000 tokens, 64
+    heads 380 / 310; 512 tokens, 64 heads 72 / 50; but sixteen sequences of 8192 tokens, 24 heads 162 / 192."""
+    seg = max(128, -(-total * units // 1024 // 16) * 16)
+    per, chunks = max(0.42, size / 128), total / 16
+    uneven = 1.0 if nseq == 1 else 1.5          # the longest sequence, whose length the host does not know, over the mean
+    walked = per * max(1.8 * uneven * chunks / nseq, 0.0101 * chunks * units)
+    cut = 10 + per * max(2.6 * seg / 16, 0.0118 * chunks * units)
+    return seg if cut < walked and total > seg * nseq and total // seg + nseq < 65535 else 0
 
 
 # ----------------------------------------------------------------------------------------- Mamba-1
@@ -276,8 +291,10 @@ def ssd_scan(x, dt, A, B, C, D=None, dt_bias=None, softplus=True, cu_seqlens=Non
         args = (x.data_ptr(), dt.data_ptr(), A.data_ptr(), B.data_ptr(), C.data_ptr(), _lib.ptr(D), _lib.ptr(dt_bias),
                 int(softplus), cu.data_ptr())
         if rec is not None:
-            _lib.call("edl_ssd_scan_chunks", *args, total, nseq, H, P, G, N, _lib.ptr(state), y.data_ptr(), rec.data_ptr(),
-                      _lib.stream_ptr())
+            seg = _scan_segment(total, nseq, H * ((P + 63) // 64), N) if state is None or state.data_ptr() % 16 == 0 else 0
+            parts = torch.empty((total // seg + nseq + 1) * H * (P * N + 1), dtype=torch.float32, device=x.device) if seg else None
+            _lib.call("edl_ssd_scan_chunks", *args, total, nseq, H, P, G, N, _lib.ptr(state), y.data_ptr(), rec.data_ptr(), seg,
+                      _lib.ptr(parts), _lib.stream_ptr())
         else:
             _lib.call("edl_ssd_scan", *args, nseq, H, P, G, N, _lib.ptr(state), y.data_ptr(), _lib.stream_ptr())
         return y

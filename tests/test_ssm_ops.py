@@ -286,3 +286,28 @@ def test_ssd_scan_many_tokens_at_a_time_matches_the_tokens_one_by_one(lens, H, P
         want = ssm.ssd_scan_reference(x.float(), dt, A, B, C, D, bias, True, cu, s2)
     assert (s1 - s2).abs().max() < 1e-5 * s2.abs().max()
     assert ((got.float() - want).abs() <= 2 ** -8 * want.abs() + 1e-5 * want.abs().max()).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("lens", [[300], [1, 47, 48, 49, 0, 16, 0, 97], [130, 0, 3, 257], [0, 161]])
+@pytest.mark.parametrize("H,P,G,N", [(4, 64, 2, 128), (3, 50, 1, 16), (6, 128, 3, 64)])
+@pytest.mark.parametrize("seg", [16, 48, 160])
+@pytest.mark.parametrize("with_state", [True, False])
+def test_ssd_segments_match_the_tokens_one_by_one(lens, H, P, G, N, seg, with_state, monkeypatch):
+    """Sequences cut into segments that run side by side: ends of segments and sequences together and apart, empty sequences,
+    with and without a state to start from."""
+    monkeypatch.setattr(ssm, "_scan_segment", lambda *a: seg)
+    torch.manual_seed(7)
+    cu, T = _tokens_of(lens)
+    bf = lambda *s: torch.randn(*s, device="cuda").to(torch.bfloat16)  # noqa: E731
+    x, dt, B, C = bf(T, H, P), bf(T, H), bf(T, G, N), bf(T, G, N)
+    A, D, bias = -4 * torch.rand(H, device="cuda"), torch.randn(H, device="cuda"), torch.randn(H, device="cuda")
+    s1 = torch.randn(len(lens), H, P, N, device="cuda") if with_state else None
+    s2 = s1.clone() if with_state else None
+    with torch.no_grad():
+        got = ssm.ssd_scan(x, dt, A, B, C, D, bias, True, cu, s1)
+        want = ssm.ssd_scan_reference(x.float(), dt, A, B, C, D, bias, True, cu, s2)
+    # fp32 sums in another order: a few 2^-24 per token; the output is rounded to bf16 (2^-9 of a value)
+    if with_state:
+        assert (s1 - s2).abs().max() < 1e-5 * s2.abs().max()
+    assert ((got.float() - want).abs() <= 2 ** -8 * want.abs() + 1e-5 * want.abs().max()).all()
