@@ -51,13 +51,13 @@ PRECISE = frozenset({"stream_ops", "hgrn2", "gdelta", "block_scan", "chunk_scan"
 
 # What serving a model family needs, by model type, for a first call on a machine without a built library.
 SERVING_PARTS = {
-    "rakevik": ("common", "gemm", "attention_fwd", "attention_decode", "attn_combine", "attention_simt", "serving",
+    "rakevik": ("common", "gemm", "gemm_skinny", "attention_fwd", "attention_decode", "attn_combine", "attention_simt", "serving",
                 "host_native", "stream_ops", "hgrn2"),
-    "disunex": ("common", "gemm", "attention_fwd", "attention_mla_decode", "attn_combine", "attention_simt", "serving",
+    "disunex": ("common", "gemm", "gemm_skinny", "attention_fwd", "attention_mla_decode", "attn_combine", "attention_simt", "serving",
                 "host_native", "stream_ops", "latent_ops", "moe", "moe_serving"),
-    "gasetar": ("common", "gemm", "attention_fwd", "attention_decode", "attention_mla_decode", "attn_combine",
+    "gasetar": ("common", "gemm", "gemm_skinny", "attention_fwd", "attention_decode", "attention_mla_decode", "attn_combine",
                 "attention_simt", "serving", "host_native", "stream_ops", "latent_ops", "moe", "moe_serving", "norm_act"),
-    "ninisun": ("common", "gemm", "attention_fwd", "attention_decode", "attn_combine", "attention_simt", "serving",
+    "ninisun": ("common", "gemm", "gemm_skinny", "attention_fwd", "attention_decode", "attn_combine", "attention_simt", "serving",
                 "host_native", "stream_ops", "gdelta", "norm_act"),
 }
 MANIFEST_SUFFIX = ".sources.json"      # beside a linked library: the digest of every source it was built from

@@ -51,3 +51,11 @@ def test_llama4_composite_is_registered_for_image_text():
     assert reg.module.__name__ == "Llama4ForConditionalGeneration"
     assert registry.get_module_registration(TaskType.BASE_VISION, "llama4_vision_model").module.__name__ == \
         "Llama4VisionModel"
+
+
+def test_partial_serving_libraries_hold_every_product_kernel():
+    """A library built with one family's parts only serves every linear that ``ops.kernels.gemm`` may choose a kernel for."""
+    from easydel_b200.csrc.build import SERVING_PARTS
+
+    for family, parts in SERVING_PARTS.items():
+        assert {"gemm", "gemm_skinny"} <= set(parts), family
