@@ -28,12 +28,14 @@ __global__ void moe_count_kernel(const long long* __restrict__ idx, long long n,
 __global__ void moe_offsets_kernel(const int* __restrict__ counts, int E, int* __restrict__ offsets,
                                    int* __restrict__ tile_expert, int max_tiles, int* __restrict__ meta,
                                    int* __restrict__ cursors) {
-  __shared__ int s_off[1025];
+  __shared__ int s_off[1025], s_count[1024];   // counts come in side by side: one after the other they took 18 us for 128
+  for (int e = threadIdx.x; e < E; e += blockDim.x) s_count[e] = counts[e];
+  __syncthreads();
   if (threadIdx.x == 0) {
     int o = 0;
     for (int e = 0; e < E; ++e) {
       s_off[e] = o;
-      o += (counts[e] + SEG - 1) / SEG * SEG;
+      o += (s_count[e] + SEG - 1) / SEG * SEG;
     }
     s_off[E] = o;
     meta[0] = o / SEG;
@@ -44,9 +46,10 @@ __global__ void moe_offsets_kernel(const int* __restrict__ counts, int E, int* _
     offsets[e] = s_off[e];
     if (e < E) cursors[e] = 0;
   }
-  for (int e = 0; e < E; ++e) {
+  const int lane = threadIdx.x & 31;
+  for (int e = threadIdx.x >> 5; e < E; e += blockDim.x >> 5) {
     const int t0 = s_off[e] / SEG, t1 = s_off[e + 1] / SEG;
-    for (int t = t0 + threadIdx.x; t < t1 && t < max_tiles; t += blockDim.x) tile_expert[t] = e;
+    for (int t = t0 + lane; t < t1 && t < max_tiles; t += 32) tile_expert[t] = e;
   }
 }
 
@@ -126,15 +129,21 @@ __global__ void moe_combine_kernel(const __nv_bfloat16* __restrict__ ys, const f
   }
 }
 
-// Backward of combine: dys[pos, :] = w[t,s] * dy[t, :] and dw[t,s] = <dy[t,:], ys[pos,:]>. One warp per pair.
-// Padding rows of dys must have been zeroed by the caller.
+// Backward of combine: dys[pos, :] = w[t,s] * dy[t, :] and dw[t,s] = <dy[t,:], ys[pos,:]>. One warp per pair, then one per row:
+// the rows that only pad a segment (no token) become zero, since the weight gradients read them; rows past the last segment
+// stay as they are, nobody reads those.
 __global__ void moe_combine_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ ys,
                                        const float* __restrict__ w, const int* __restrict__ slot_pos,
                                        __nv_bfloat16* __restrict__ dys, float* __restrict__ dw, long long pairs, int k,
-                                       int H) {
+                                       int H, const int* __restrict__ row_token, const int* __restrict__ meta) {
   const long long wid = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
-  if (wid >= pairs) return;
+  if (wid >= pairs) {
+    const long long row = wid - pairs;
+    if (row < meta[1] && row_token[row] < 0)
+      for (int c = lane * 8; c < H; c += 256) *reinterpret_cast<uint4*>(dys + row * H + c) = make_uint4(0u, 0u, 0u, 0u);
+    return;
+  }
   const int pos = slot_pos[wid];
   if (pos < 0) {
     if (lane == 0 && dw) dw[wid] = 0.f;
@@ -241,13 +250,16 @@ EDL_HOST_API int edl_moe_combine(const void* ys, const float* w, const int* slot
   return check_cuda(cudaGetLastError(), "moe_combine launch");
 }
 
+// row_token, meta: of edl_moe_route, over max_rows rows of dys.
 EDL_HOST_API int edl_moe_combine_bwd(const void* dy, const void* ys, const float* w, const int* slot_pos, void* dys,
-                                     float* dw, long long T, int k, int H, void* stream) {
+                                     float* dw, long long T, int k, int H, const int* row_token, const int* meta,
+                                     long long max_rows, void* stream) {
   if (T <= 0) return 0;
   const long long pairs = T * k;
-  const long long blocks = (pairs * 32 + 255) / 256;
+  const long long blocks = ((pairs + max_rows) * 32 + 255) / 256;
   moe_combine_bwd_kernel<<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(
-      (const __nv_bfloat16*)dy, (const __nv_bfloat16*)ys, w, slot_pos, (__nv_bfloat16*)dys, dw, pairs, k, H);
+      (const __nv_bfloat16*)dy, (const __nv_bfloat16*)ys, w, slot_pos, (__nv_bfloat16*)dys, dw, pairs, k, H, row_token,
+      meta);
   return check_cuda(cudaGetLastError(), "moe_combine_bwd launch");
 }
 

@@ -212,9 +212,11 @@ __device__ __forceinline__ float act_grad(float x, int act) {
   }
 }
 
+// rows: where there is one, the number of rows in use, on the device (the expert rows of a routed batch).
 __global__ void gated_act_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ h, long long T,
-                                     int F, long long ld_gu, int act) {
+                                     int F, long long ld_gu, int act, const int* __restrict__ rows) {
   const int vecs = F / 8;
+  if (rows) T = min(T, (long long)*rows);
   long long total = T * vecs;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
        i += (long long)gridDim.x * blockDim.x) {
@@ -229,9 +231,12 @@ __global__ void gated_act_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_
   }
 }
 
+// h: where there is one, the forward's output is written again beside the gradient (gate and up are here anyway).
 __global__ void gated_act_bwd_kernel(const __nv_bfloat16* __restrict__ gu, const __nv_bfloat16* __restrict__ dh,
-                                     __nv_bfloat16* __restrict__ dgu, long long T, int F, long long ld_gu, int act) {
+                                     __nv_bfloat16* __restrict__ dgu, long long T, int F, long long ld_gu, int act,
+                                     const int* __restrict__ rows, __nv_bfloat16* __restrict__ h) {
   const int vecs = F / 8;
+  if (rows) T = min(T, (long long)*rows);
   long long total = T * vecs;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
        i += (long long)gridDim.x * blockDim.x) {
@@ -244,10 +249,13 @@ __global__ void gated_act_bwd_kernel(const __nv_bfloat16* __restrict__ gu, const
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       dg[j] = d[j] * u[j] * act_grad(g[j], act);
-      du[j] = d[j] * act_fwd(g[j], act);
+      const float a = act_fwd(g[j], act);
+      du[j] = d[j] * a;
+      u[j] *= a;
     }
     store8(dgu + t * ld_gu + c, dg);
     store8(dgu + t * ld_gu + F + c, du);
+    if (h) store8(h + t * F + c, u);
   }
 }
 
@@ -474,8 +482,33 @@ EDL_HOST_API int edl_gated_act_fwd(const void* gu, void* h, long long T, int F, 
     return -1;
   }
   gated_act_fwd_kernel<<<grid_for(T * (F / 8), 256), 256, 0, (cudaStream_t)stream>>>(
-      (const __nv_bfloat16*)gu, (__nv_bfloat16*)h, T, F, ld_gu, act);
+      (const __nv_bfloat16*)gu, (__nv_bfloat16*)h, T, F, ld_gu, act, nullptr);
   return check_cuda(cudaGetLastError(), "gated_act_fwd launch");
+}
+// The same over the first *rows of max_rows rows [gate | up] without a pitch.
+EDL_HOST_API int edl_gated_act_rows_fwd(const void* gu, void* h, long long max_rows, const int* rows, int F, int act,
+                                        void* stream) {
+  if (max_rows <= 0) return 0;
+  if (F % 8 || !rows) {
+    set_last_error("edl_gated_act_rows_fwd: F must be a multiple of 8");
+    return -1;
+  }
+  gated_act_fwd_kernel<<<grid_for(max_rows * (F / 8), 256), 256, 0, (cudaStream_t)stream>>>(
+      (const __nv_bfloat16*)gu, (__nv_bfloat16*)h, max_rows, F, 2LL * F, act, rows);
+  return check_cuda(cudaGetLastError(), "gated_act_rows_fwd launch");
+}
+// dgu from dh, and the forward's output h again.
+EDL_HOST_API int edl_gated_act_rows_bwd(const void* gu, const void* dh, void* dgu, void* h, long long max_rows,
+                                        const int* rows, int F, int act, void* stream) {
+  if (max_rows <= 0) return 0;
+  if (F % 8 || !rows) {
+    set_last_error("edl_gated_act_rows_bwd: F must be a multiple of 8");
+    return -1;
+  }
+  gated_act_bwd_kernel<<<grid_for(max_rows * (F / 8), 256), 256, 0, (cudaStream_t)stream>>>(
+      (const __nv_bfloat16*)gu, (const __nv_bfloat16*)dh, (__nv_bfloat16*)dgu, max_rows, F, 2LL * F, act, rows,
+      (__nv_bfloat16*)h);
+  return check_cuda(cudaGetLastError(), "gated_act_rows_bwd launch");
 }
 
 EDL_HOST_API int edl_gated_act_bwd(const void* gu, const void* dh, void* dgu, long long T, int F, long long ld_gu,
@@ -486,7 +519,8 @@ EDL_HOST_API int edl_gated_act_bwd(const void* gu, const void* dh, void* dgu, lo
     return -1;
   }
   gated_act_bwd_kernel<<<grid_for(T * (F / 8), 256), 256, 0, (cudaStream_t)stream>>>(
-      (const __nv_bfloat16*)gu, (const __nv_bfloat16*)dh, (__nv_bfloat16*)dgu, T, F, ld_gu, act);
+      (const __nv_bfloat16*)gu, (const __nv_bfloat16*)dh, (__nv_bfloat16*)dgu, T, F, ld_gu, act, nullptr,
+      nullptr);
   return check_cuda(cudaGetLastError(), "gated_act_bwd launch");
 }
 

@@ -15,7 +15,9 @@ vp, i32, i64 = _lib.vp, _lib.i32, _lib.i64
 _lib.register("edl_moe_route", i32, [vp, i64, i32, i32, i32, vp, vp, vp, vp, i32, vp, vp, vp, vp])
 _lib.register("edl_moe_gather", i32, [vp, vp, vp, vp, i32, i64, i64, vp])
 _lib.register("edl_moe_combine", i32, [vp, vp, vp, vp, i64, i32, i32, i32, vp])
-_lib.register("edl_moe_combine_bwd", i32, [vp, vp, vp, vp, vp, vp, i64, i32, i32, vp])
+_lib.register("edl_moe_combine_bwd", i32, [vp, vp, vp, vp, vp, vp, i64, i32, i32, vp, vp, i64, vp])
+_lib.register("edl_gated_act_rows_fwd", i32, [vp, vp, i64, vp, i32, i32, vp])
+_lib.register("edl_gated_act_rows_bwd", i32, [vp, vp, vp, vp, i64, vp, i32, i32, vp])
 _lib.register("edl_moe_gather_bwd", i32, [vp, vp, vp, i64, i32, i32, vp])
 _lib.register("edl_gemm_grouped", i32, [i32, vp, vp, vp, vp, i32, i32, i32, i32, vp, vp, vp, i32, vp, vp])
 
@@ -62,16 +64,16 @@ class Routing:
         return out
 
 
-def _grouped_fwd(r: Routing, xs: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
+def _grouped_fwd(r: Routing, xs: torch.Tensor, w: torch.Tensor, defined: bool = True) -> torch.Tensor:
     E, N, Kd = w.shape
-    # rows past the last segment are never written: start from zeros so later passes read defined values
-    out = torch.zeros(r.max_rows, N, dtype=xs.dtype, device=xs.device)
+    # rows past the last segment are never written: ``defined`` starts from zeros for passes that read them
+    out = (torch.zeros if defined else torch.empty)(r.max_rows, N, dtype=xs.dtype, device=xs.device)
     return r.grouped(0, xs, w, out, N=N, Kd=Kd)
 
 
-def _grouped_dgrad(r: Routing, dy: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
+def _grouped_dgrad(r: Routing, dy: torch.Tensor, w: torch.Tensor, defined: bool = True) -> torch.Tensor:
     E, N, Kd = w.shape
-    out = torch.zeros(r.max_rows, Kd, dtype=dy.dtype, device=dy.device)
+    out = (torch.zeros if defined else torch.empty)(r.max_rows, Kd, dtype=dy.dtype, device=dy.device)
     return r.grouped(1, dy, w, out, N=N, Kd=Kd)
 
 
@@ -83,15 +85,20 @@ def _grouped_wgrad(r: Routing, dy: torch.Tensor, xs: torch.Tensor, out: torch.Te
 
 
 class _MoEFFN(torch.autograd.Function):
+    """Every pass here goes over the rows in use (``meta[1]``, on the device), so the row buffers start undefined: filling them
+    took 0.22 ms of 2.8 at 4096 tokens, 128 experts of 2048 x 768."""
+
     @staticmethod
     def forward(ctx, x, w_gu, w_d, topk_w, topk_idx, act, expert_offset):
         T, H = x.shape
         k = topk_idx.shape[1]
         r = Routing(topk_idx, w_gu.shape[0], expert_offset)
         xs = r.gather(x)
-        h = _grouped_fwd(r, xs, w_gu)
-        a = K.gated_act_fwd(h, act)
-        ys = _grouped_fwd(r, a, w_d)
+        h = _grouped_fwd(r, xs, w_gu, defined=False)
+        a = torch.empty(r.max_rows, h.shape[1] // 2, dtype=h.dtype, device=h.device)
+        _lib.call("edl_gated_act_rows_fwd", h.data_ptr(), a.data_ptr(), r.max_rows, r.meta[1:].data_ptr(), a.shape[1],
+                  K.ACT_IDS[act], _lib.stream_ptr())
+        ys = _grouped_fwd(r, a, w_d, defined=False)
         wf = topk_w.to(torch.float32).contiguous()
         y = torch.empty(T, H, dtype=x.dtype, device=x.device)
         _lib.call("edl_moe_combine", ys.data_ptr(), wf.data_ptr(), r.slot_pos.data_ptr(), y.data_ptr(), T, k, H, 0,
@@ -106,12 +113,15 @@ class _MoEFFN(torch.autograd.Function):
         r, act = ctx.r, ctx.act
         T, H, k = ctx.shape
         dy = dy.contiguous()
-        dys = torch.zeros_like(ys)
+        dys = torch.empty_like(ys)
         dwr = torch.empty(T, k, dtype=torch.float32, device=dy.device)
         _lib.call("edl_moe_combine_bwd", dy.data_ptr(), ys.data_ptr(), wf.data_ptr(), r.slot_pos.data_ptr(),
-                  dys.data_ptr(), dwr.data_ptr(), T, k, H, _lib.stream_ptr())
-        a = K.gated_act_fwd(h, act)
-        da = _grouped_dgrad(r, dys, w_d)
+                  dys.data_ptr(), dwr.data_ptr(), T, k, H, r.row_token.data_ptr(), r.meta.data_ptr(), r.max_rows,
+                  _lib.stream_ptr())
+        da = _grouped_dgrad(r, dys, w_d, defined=False)
+        a, dh = torch.empty_like(da), torch.empty_like(h)
+        _lib.call("edl_gated_act_rows_bwd", h.data_ptr(), da.data_ptr(), dh.data_ptr(), a.data_ptr(), r.max_rows,
+                  r.meta[1:].data_ptr(), a.shape[1], K.ACT_IDS[act], _lib.stream_ptr())
         g_wd = g_wgu = None
         for w, dyv, xin, name in ((w_d, dys, a, "d"), (None, None, None, None)):
             if w is None:
@@ -125,7 +135,6 @@ class _MoEFFN(torch.autograd.Function):
                     buf = torch.zeros(w.shape, dtype=torch.float32, device=dy.device)
                     _grouped_wgrad(r, dyv, xin, buf, False)
                     g_wd = buf.to(w.dtype)
-        dh = K.gated_act_bwd(h, da, act)
         if ctx.needs_input_grad[1]:
             mg = getattr(w_gu, "main_grad", None)
             if mg is not None:
@@ -137,7 +146,7 @@ class _MoEFFN(torch.autograd.Function):
                 g_wgu = buf.to(w_gu.dtype)
         dx = None
         if ctx.needs_input_grad[0]:
-            dxs = _grouped_dgrad(r, dh, w_gu)
+            dxs = _grouped_dgrad(r, dh, w_gu, defined=False)
             dx = torch.empty(T, H, dtype=dy.dtype, device=dy.device)
             _lib.call("edl_moe_gather_bwd", dxs.data_ptr(), r.slot_pos.data_ptr(), dx.data_ptr(), T, k, H,
                       _lib.stream_ptr())

@@ -83,3 +83,27 @@ def test_moe_ffn_with_expert_biases_and_gptoss_gate():
     for a, b, name in zip(dev, cpu, ("dx", "dW_gate_up", "dW_down", "dw", "db_gate_up", "db_down")):
         rel = ((a.grad.float().cpu() - b.grad).norm() / (b.grad.norm() + 1e-8)).item()
         assert rel < 0.05, f"{name}: {rel}"
+
+
+@pytest.mark.parametrize("T,E,k", [(1, 4, 1), (130, 8, 2), (300, 3, 3)])
+def test_moe_ffn_reads_no_undefined_rows(T, E, k):
+    """Row buffers start undefined: with NaN in all fresh memory, outputs and every gradient equal those from clean memory."""
+    from easydel_b200.ops.moe_kernels import moe_ffn
+
+    torch.manual_seed(T)
+    H, Fd = 128, 96
+    mk = lambda *s: (torch.randn(*s, device="cuda") * 0.1).to(torch.bfloat16)  # noqa: E731
+    x0, gu0, d0, dy = mk(T, H), mk(E, 2 * Fd, H), mk(E, H, Fd), mk(T, H)
+    p0, idx = torch.softmax(torch.randn(T, E, device="cuda"), -1).topk(k, -1)
+    got = []
+    for fill in (0.0, float("nan")):
+        torch.cuda.empty_cache()
+        junk = [torch.full((1 << 22,), fill, device="cuda") for _ in range(24)]
+        del junk                       # the allocator hands these blocks out again
+        x, gu, d, p = (t.clone().requires_grad_() for t in (x0, gu0, d0, p0))
+        y = moe_ffn(x, gu, d, p, idx)
+        got.append([y.detach(), *torch.autograd.grad(y, [x, gu, d, p], dy)])
+    for a, b in zip(*got):
+        assert torch.isfinite(a.float()).all()
+        # pairs meet an expert in any order, which changes the order of sums over rows
+        assert (a.float() - b.float()).abs().max() <= 2.0 ** -7 * a.float().abs().max()
