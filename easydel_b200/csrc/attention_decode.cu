@@ -5,12 +5,12 @@
 // attention_fwd.cu processes a sequence as one 128-row tile with a two-stage ring and spends microseconds per
 // 128-key step on a tile that holds G real rows; this kernel is the streaming form:
 //
-//   * one CTA per (sequence, KV head, key split); its four warps take 32-key tiles round-robin, each warp with its
+//   * one CTA per (sequence, KV head, key split); its two or four warps take 32-key tiles round-robin, each warp with its
 //     own three-stage ring of [32 keys x D] K and V tiles filled by TMA (lane 0 issues, an mbarrier per stage
-//     receives the bytes), so 4 x 2 x 16 KB are in flight per CTA without any CTA-wide synchronisation;
+//     receives the bytes), so 4 x 2 x 16 KB are in flight per SM without any CTA-wide synchronisation;
 //   * scores and the weighted value sum run on the tensor cores as m16n8k16 bf16 products (the G <= 16 query rows
 //     are the M side; the 5th-generation MMA path has no shape this small, and the kernel is bandwidth bound);
-//   * every warp keeps an online softmax for its keys; at the end the four partial (max, sum, O) triples are merged
+//   * every warp keeps an online softmax for its keys; at the end the partial (max, sum, O) triples of the warps are merged
 //     through shared memory and written as bf16 rows, plus the log-sum-exp when the caller merges key splits.
 //
 // Replaces the decode branch of the reference's ragged / paged attention kernels
@@ -22,15 +22,7 @@
 namespace edl {
 namespace {
 
-#ifndef EDL_DEC_WARPS
-#define EDL_DEC_WARPS 4
-#endif
-#ifndef EDL_DEC_TK
-#define EDL_DEC_TK 32
-#endif
-constexpr int DEC_WARPS = EDL_DEC_WARPS;
-constexpr int DEC_THREADS = DEC_WARPS * 32;
-constexpr int TK = EDL_DEC_TK;        // keys per tile (16 or 32)
+constexpr int TK = 32;                // keys per tile
 constexpr int DEC_STAGES = 3;
 constexpr int PAGE = 128;
 constexpr float LOG2E_F = 1.4426950408889634f;
@@ -82,7 +74,7 @@ __device__ __forceinline__ uint32_t tile_off(int row, int chunk) {
   return box * (TK * 128) + row * 128 + ((c ^ (row & 7)) << 4);
 }
 
-template <int DQ, int DV>
+template <int DQ, int DV, int DEC_WARPS>
 struct DCfg {
   static constexpr int K_BYTES = TK * DQ * 2;                         // one K tile
   static constexpr int STAGE_BYTES = K_BYTES + TK * DV * 2;           // K + V
@@ -94,11 +86,12 @@ struct DCfg {
   static constexpr int SMEM = OFF_RED + DEC_WARPS * 2 * 16 * 4 + 1024;
 };
 
-template <int DQ, int DV, bool SIG>
-__global__ void __launch_bounds__(DEC_THREADS)
+template <int DQ, int DV, bool SIG, int DEC_WARPS>
+__global__ void __launch_bounds__(DEC_WARPS * 32)
 attn_decode_kernel(const __grid_constant__ CUtensorMap tk, const __grid_constant__ CUtensorMap tv,
                    const DecodeParams p) {
-  using C = DCfg<DQ, DV>;
+  using C = DCfg<DQ, DV, DEC_WARPS>;
+  constexpr int DEC_THREADS = DEC_WARPS * 32;
   constexpr int NKS = DQ / 16;     // k-steps of the score product
   constexpr int NDB = DV / 8;     // 8-column blocks of the output
   constexpr int QPITCH = DQ * 2 + 16;
@@ -126,7 +119,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tk, const __grid_constant
   const int t0 = split * per_split;
   const int t1 = min(n_all, t0 + per_split);
   const int n_tiles = max(0, t1 - t0);
-  // places of this warp: t0 + warp, t0 + warp + 4, ...
+  // places of this warp: t0 + warp, t0 + warp + DEC_WARPS, ...
   const int my_n = n_tiles > warp ? (n_tiles - warp + DEC_WARPS - 1) / DEC_WARPS : 0;
 
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::OFF_BAR);
@@ -211,20 +204,22 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tk, const __grid_constant
     const int key0 = tile * TK;
 
     // ---- S = Q K^T for 32 keys: four 8-key blocks
+    // the key blocks take turns: one block's chain of products alone would wait for each of them
     float s[TK / 8][4];
 #pragma unroll
-    for (int j = 0; j < TK / 8; ++j) {
+    for (int j = 0; j < TK / 8; ++j)
 #pragma unroll
       for (int e = 0; e < 4; ++e) s[j][e] = 0.f;
 #pragma unroll
-      for (int ks = 0; ks < NKS; ks += 2) {
-        // four matrices of key block j: d-chunks 2ks, 2ks+1 (k-step ks) and 2ks+2, 2ks+3 (k-step ks+1)
-        uint32_t kb[4];
-        const int row = j * 8 + (lane & 7);
-        ldmatrix_x4(kt + tile_off(row, ks * 2 + (lane >> 3)), kb);
-        mma_bf16_16816(s[j], qa[ks], kb[0], kb[1]);
-        mma_bf16_16816(s[j], qa[ks + 1], kb[2], kb[3]);
-      }
+    for (int ks = 0; ks < NKS; ks += 2) {
+      // four matrices per key block: d-chunks 2ks, 2ks+1 (k-step ks) and 2ks+2, 2ks+3 (k-step ks+1)
+      uint32_t kb[TK / 8][4];
+#pragma unroll
+      for (int j = 0; j < TK / 8; ++j) ldmatrix_x4(kt + tile_off(j * 8 + (lane & 7), ks * 2 + (lane >> 3)), kb[j]);
+#pragma unroll
+      for (int j = 0; j < TK / 8; ++j) mma_bf16_16816(s[j], qa[ks], kb[j][0], kb[j][1]);
+#pragma unroll
+      for (int j = 0; j < TK / 8; ++j) mma_bf16_16816(s[j], qa[ks + 1], kb[j][2], kb[j][3]);
     }
     // ---- mask the ragged end / the window start, online softmax (log2 domain)
     const int cbase = key0 + (lane & 3) * 2;
@@ -287,12 +282,14 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tk, const __grid_constant
       l_run[0] += rs[0];
       l_run[1] += rs[1];
       // ---- O = O * alpha + P V
+      if (__any_sync(0xffffffffu, alpha[0] != 1.f || alpha[1] != 1.f)) {   // most tiles raise no row's maximum
 #pragma unroll
-      for (int j = 0; j < NDB; ++j) {
-        o_acc[j][0] *= alpha[0];
-        o_acc[j][1] *= alpha[0];
-        o_acc[j][2] *= alpha[1];
-        o_acc[j][3] *= alpha[1];
+        for (int j = 0; j < NDB; ++j) {
+          o_acc[j][0] *= alpha[0];
+          o_acc[j][1] *= alpha[0];
+          o_acc[j][2] *= alpha[1];
+          o_acc[j][3] *= alpha[1];
+        }
       }
     }
 #pragma unroll
@@ -317,7 +314,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tk, const __grid_constant
     l_run[h] += __shfl_xor_sync(0xffffffffu, l_run[h], 2);
   }
 
-  // ---- merge the four warps: (m, l) through shared memory, O through the (now idle) tile rings
+  // ---- merge the warps: (m, l) through shared memory, O through the (now idle) tile rings
   float* red = reinterpret_cast<float*>(smem + C::OFF_RED);   // [warp][m 16 | l 16]
   const int r0 = lane >> 2;
   if ((lane & 3) == 0) {
@@ -429,15 +426,15 @@ __global__ void sum_parts_kernel(const float* __restrict__ parts, int splits, in
   }
 }
 
-template <int DQ, int DV, bool SIG>
-int launch_decode(const void* k_pages, const void* v_pages, long long ld_kpage, long long ld_vpage,
+template <int DQ, int DV, bool SIG, int DEC_WARPS>
+int launch_decode_as(const void* k_pages, const void* v_pages, long long ld_kpage, long long ld_vpage,
                   long long num_pages, const DecodeParams& p, cudaStream_t stream) {
-  using C = DCfg<DQ, DV>;
+  using C = DCfg<DQ, DV, DEC_WARPS>;
   CUtensorMap tk, tv;
   const long long total_k = num_pages * PAGE;
   if (make_tmap_3d_16b(&tk, k_pages, p.dq, p.Hkv, total_k, p.dq, ld_kpage, 64, 1, TK, 3)) return -1;
   if (make_tmap_3d_16b(&tv, v_pages, p.dv, p.Hkv, total_k, p.dv, ld_vpage, 64, 1, TK, 3)) return -1;
-  auto kern = attn_decode_kernel<DQ, DV, SIG>;
+  auto kern = attn_decode_kernel<DQ, DV, SIG, DEC_WARPS>;
   static bool attr_set[64] = {false};
   int dev = 0;
   cudaGetDevice(&dev);
@@ -449,13 +446,30 @@ int launch_decode(const void* k_pages, const void* v_pages, long long ld_kpage, 
     attr_set[dev] = true;
   }
   const long long blocks = (long long)p.B * p.Hkv * p.splits;
-  kern<<<(unsigned)blocks, DEC_THREADS, C::SMEM, stream>>>(tk, tv, p);
+  kern<<<(unsigned)blocks, DEC_WARPS * 32, C::SMEM, stream>>>(tk, tv, p);
   if (SIG && p.splits > 1) {
     const int width = p.Hq * p.dv;
     const long long n = (long long)p.B * (width / 4);
     sum_parts_kernel<<<(int)((n + 255) / 256), 256, 0, stream>>>(p.parts, p.splits, p.B, width, p.o, p.ldo);
   }
   return check_cuda(cudaGetLastError(), "attn_decode launch");
+}
+
+// CTAs of two warps leave room for another one on their SM, whose loads run while this one starts and merges; CTAs of four
+// finish a sequence in half the time. Counted in rounds of resident CTAs, a round of two-warp CTAs taking twice as long but
+// for the start (half of a four-warp round's keys). One B200, 128-wide heads, us, four / two warps: 256 sequences of 420 to
+// 1400 keys, 8 KV heads (2048 CTAs) 194.6 / 161.0 (147 at the copy rate); 512 CTAs 33.0 / 24.8; 256 CTAs 24.7 / 23.0; 384
+// CTAs 73.1 / 81.9; 128 CTAs 34.8 / 57.6.
+template <int DQ, int DV, bool SIG>
+int launch_decode(const void* k_pages, const void* v_pages, long long ld_kpage, long long ld_vpage, long long num_pages,
+                  const DecodeParams& p, cudaStream_t stream) {
+  constexpr int SM_BYTES = 227 * 1024, KERNEL_BYTES = 1024;
+  const long long ctas = (long long)p.B * p.Hkv * p.splits, sms = sm_count();
+  const long long at4 = sms * (SM_BYTES / (DCfg<DQ, DV, 4>::SMEM + KERNEL_BYTES)), at2 = sms * (SM_BYTES / (DCfg<DQ, DV, 2>::SMEM + KERNEL_BYTES));
+  const long long rounds4 = (ctas + at4 - 1) / at4, rounds2 = (ctas + at2 - 1) / at2;
+  return 5 * rounds2 < 3 * rounds4
+             ? launch_decode_as<DQ, DV, SIG, 2>(k_pages, v_pages, ld_kpage, ld_vpage, num_pages, p, stream)
+             : launch_decode_as<DQ, DV, SIG, 4>(k_pages, v_pages, ld_kpage, ld_vpage, num_pages, p, stream);
 }
 
 template <bool SIG>

@@ -209,6 +209,37 @@ def test_latent_decode_attention_kernel(B, H, ctx, splits):
         assert err < 2e-2, (b, float(err))
 
 
+@pytest.mark.parametrize("D,Dv,window,softcap", [(128, 128, 0, 0.0), (128, 64, 50, 0.0), (72, 128, 0, 5.0), (64, 64, 33, 0.0)])
+def test_decode_attention_with_more_sequences_than_sms(D, Dv, window, softcap):
+    """Enough (sequence, KV head) pairs for two CTAs per SM, which have two warps each: lengths around a tile of 32 keys and a
+    round of two tiles, one key only, several pages."""
+    from easydel_b200.ops import serving as S
+
+    torch.manual_seed(0)
+    lens = [1, 31, 32, 33, 63, 64, 65, 127, 128, 129, 300] * 40
+    B, Hkv, G = len(lens), 3, 4
+    per = 3
+    kp = torch.randn(B * per + 1, 128, Hkv, D, device="cuda").to(torch.bfloat16)
+    vp = torch.randn(B * per + 1, 128, Hkv, Dv, device="cuda").to(torch.bfloat16)
+    table = (torch.randperm(B * per, device="cuda") + 1).view(B, per).to(torch.int32)
+    q = torch.randn(B, Hkv * G, D, device="cuda").to(torch.bfloat16)
+    sinks = torch.randn(Hkv * G, device="cuda")
+    kv = torch.tensor(lens, dtype=torch.int32, device="cuda")
+    o = S.decode_attention(q, kp, vp, kv, table, window=window, sinks=sinks, softcap=softcap)
+    k = kp[table.long()].reshape(B, -1, Hkv, D).double().repeat_interleave(G, 2)
+    v = vp[table.long()].reshape(B, -1, Hkv, Dv).double().repeat_interleave(G, 2)
+    s = torch.einsum("bhd,bkhd->bhk", q.double(), k) * D ** -0.5
+    if softcap:
+        s = softcap * torch.tanh(s / softcap)
+    at = torch.arange(per * 128, device="cuda")[None]
+    see = (at < kv[:, None]) & (at >= kv[:, None] - (window or per * 128))
+    s = s.masked_fill(~see[:, None], float("-inf"))
+    p = torch.softmax(torch.cat([s, sinks.double()[None, :, None].expand(B, -1, 1)], -1), -1)[..., :-1]
+    want = torch.einsum("bhk,bkhd->bhd", p, v)
+    # probabilities and outputs are rounded to bf16: 2^-9 each of the largest value of a row
+    assert (o.double() - want).abs().max() <= 3 * 2.0 ** -9 * v.abs().max()
+
+
 @pytest.mark.parametrize("H,L,R", [(17, 512, 64), (64, 512, 64), (128, 512, 64), (130, 512, 64), (40, 128, 64), (33, 320, 32),
                                    (20, 72, 24), (18, 504, 72), (24, 256, 0), (5, 512, 64)])
 @pytest.mark.parametrize("lens", [[1], [64, 65, 0, 700, 129], [33] * 20 + [2000], [190] * 90])
