@@ -5,7 +5,7 @@ layers/linears/_linear_quantized.py): ``int8`` (symmetric), ``affine`` 4 / 8 bit
 (normal-float code book, absmax per block), ``mxfp4`` / ``mxfp8`` (e2m1 / e4m3 values with a power-of-two scale per
 32), ``nvfp4`` (e2m1 with an e4m3 scale per 16) and ``nvfp8`` (e4m3 with one scale per row). All of them are stored
 as ``codes`` + per-group ``scales`` (+ ``zeros``) + a code book, which is what ``csrc/quant.cu`` consumes:
-decode steps (up to 8 rows) run the fused dequant-GEMV, larger batches dequantise into bf16 and use the tcgen05 GEMM.
+decode steps (up to 16 rows) run the fused product, larger batches dequantise into bf16 and use the tcgen05 GEMM.
 """
 
 from __future__ import annotations
@@ -193,6 +193,7 @@ def quantize(w: torch.Tensor, config: EasyDeLQuantizationConfig | str = "nf4") -
 
 
 QGEMV_ROWS = 16      # rows up to which the fused product is the faster one
+QGEMV_INPUTS = 47104     # inputs of 16 rows that its shared memory holds over a cluster; twice as many of 8 rows
 
 
 def quantized_matmul(x: torch.Tensor, q: QuantizedTensor, bias: torch.Tensor | None = None) -> torch.Tensor:
@@ -202,7 +203,7 @@ def quantized_matmul(x: torch.Tensor, q: QuantizedTensor, bias: torch.Tensor | N
     M = x2.shape[0]
     per16 = 32 if q.bits == 4 else 16
     if x2.is_cuda and _lib.available() and x2.dtype == torch.bfloat16:
-        if M <= QGEMV_ROWS and q.group % per16 == 0:
+        if M <= QGEMV_ROWS and q.group % per16 == 0 and K <= QGEMV_INPUTS * (2 if M <= 8 else 1):
             if x2.stride(1) != 1 or x2.stride(0) % 8 or x2.data_ptr() % 16:
                 x2 = x2.clone(memory_format=torch.contiguous_format)
             out = torch.empty(M, N, dtype=torch.bfloat16, device=x.device)

@@ -45,6 +45,19 @@ def test_quantizer_replaces_linears_and_keeps_outputs_close():
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("fmt", ["nf4", "int8"])
+@pytest.mark.parametrize("K,M", [(47104, 16), (47232, 16), (94208, 8), (94336, 8), (94336, 1)])
+def test_products_at_the_limit_of_shared_memory(fmt, K, M):
+    torch.manual_seed(0)
+    block = 64 if fmt == "nf4" else 128
+    q = quantize(torch.randn(24, K, device="cuda") * 0.05, EasyDeLQuantizationConfig(fmt, block_size=block))
+    x = torch.randn(M, K, device="cuda").to(torch.bfloat16)
+    ref = x.double() @ dequantize_reference(q).double().t()
+    # above the limit weights are rounded to bf16 first: 2^-9 of each product, adding up as a random walk
+    assert (quantized_matmul(x, q).double() - ref).abs().max() <= 2.0 ** -7 * ref.abs().max()
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("fmt,block", [("nf4", 64), ("nf4", 128), ("nf4", 96), ("affine", 32), ("a4bit", 64), ("mxfp4", None),
                                        ("int8", 128), ("int8", 48), ("a8bit", 32), ("mxfp8", None), ("nvfp8", None)])
 @pytest.mark.parametrize("N,K", [(5, 96), (17, 288), (130, 1152), (1000, 6240)])
