@@ -38,7 +38,9 @@ __device__ __forceinline__ void store8(__nv_bfloat16* p, const float (&f)[8]) {
 //   residual or x) and normalised; else h = x.
 //   y = h * rsqrt(mean(h^2) + eps) * (w + w_offset)   (w_offset = 1 for Gemma)
 // ---------------------------------------------------------------------------
-template <int MAX_VEC>  // vectors of 8 per thread kept in registers
+// EARLY: the weights come with the row; behind the sum they are one more trip to memory (48 rows of 4096: 3.2 -> 2.7 us). With
+// many rows per SM that trip is hidden and the registers are missed (8192 rows: 53 against 62 us).
+template <int MAX_VEC, bool EARLY>  // vectors of 8 per thread kept in registers
 __global__ void __launch_bounds__(NORM_THREADS)
 rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* residual, const __nv_bfloat16* __restrict__ w,
                    __nv_bfloat16* __restrict__ y, __nv_bfloat16* res_out, float* __restrict__ rstd_out, int rows, int D,
@@ -48,15 +50,14 @@ rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* res
   for (int row = blockIdx.x; row < rows; row += gridDim.x) {
     const __nv_bfloat16* xr = x + (size_t)row * D;
     float h[MAX_VEC][8];
-    uint4 wv[MAX_VEC];      // the weights come with the row: behind the sum they were one more trip to memory
-                            // (1 row of 4096: 4.1 -> 3.7 us)
+    uint4 wv[EARLY ? MAX_VEC : 1];
     float ss = 0.f;
 #pragma unroll
     for (int i = 0; i < MAX_VEC; ++i) {
       int vi = threadIdx.x + i * NORM_THREADS;
       if (vi < nvec) {
         load8(xr + vi * 8, h[i]);
-        wv[i] = *reinterpret_cast<const uint4*>(w + vi * 8);
+        if constexpr (EARLY) wv[i] = *reinterpret_cast<const uint4*>(w + vi * 8);
         if (residual) {
           float r[8];
           load8(residual + (size_t)row * D + vi * 8, r);
@@ -86,7 +87,8 @@ rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* res
       int vi = threadIdx.x + i * NORM_THREADS;
       if (vi < nvec) {
         float o[8];
-        const uint32_t ww[4] = {wv[i].x, wv[i].y, wv[i].z, wv[i].w};
+        const uint4 wq = EARLY ? wv[EARLY ? i : 0] : *reinterpret_cast<const uint4*>(w + vi * 8);
+        const uint32_t ww[4] = {wq.x, wq.y, wq.z, wq.w};
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           const float2 f = unpack_bf16x2(ww[j]);
@@ -431,14 +433,17 @@ EDL_HOST_API int edl_rmsnorm_fwd(const void* x, const void* residual, const void
   auto Y = (__nv_bfloat16*)y;
   auto RO = (__nv_bfloat16*)res_out;
   int nvec = D / 8;
-  if (nvec <= NORM_THREADS)
-    rmsnorm_fwd_kernel<1><<<grid, NORM_THREADS, 0, s>>>(X, R, W, Y, RO, rstd, rows, D, eps, w_offset);
-  else if (nvec <= 2 * NORM_THREADS)
-    rmsnorm_fwd_kernel<2><<<grid, NORM_THREADS, 0, s>>>(X, R, W, Y, RO, rstd, rows, D, eps, w_offset);
-  else if (nvec <= 4 * NORM_THREADS)
-    rmsnorm_fwd_kernel<4><<<grid, NORM_THREADS, 0, s>>>(X, R, W, Y, RO, rstd, rows, D, eps, w_offset);
-  else
-    rmsnorm_fwd_kernel<8><<<grid, NORM_THREADS, 0, s>>>(X, R, W, Y, RO, rstd, rows, D, eps, w_offset);
+  const bool early = rows <= 2 * sm_count();
+#define EDL_NORM(VECS)                                                                                                      \
+  do {                                                                                                                      \
+    if (early) rmsnorm_fwd_kernel<VECS, true><<<grid, NORM_THREADS, 0, s>>>(X, R, W, Y, RO, rstd, rows, D, eps, w_offset);   \
+    else rmsnorm_fwd_kernel<VECS, false><<<grid, NORM_THREADS, 0, s>>>(X, R, W, Y, RO, rstd, rows, D, eps, w_offset);        \
+  } while (0)
+  if (nvec <= NORM_THREADS) EDL_NORM(1);
+  else if (nvec <= 2 * NORM_THREADS) EDL_NORM(2);
+  else if (nvec <= 4 * NORM_THREADS) EDL_NORM(4);
+  else EDL_NORM(8);
+#undef EDL_NORM
   return check_cuda(cudaGetLastError(), "rmsnorm_fwd launch");
 }
 
