@@ -468,7 +468,7 @@ mla_decode_tc_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_cons
     if (n > 0) {
       const int row = row_of(0);
       load_own(0, row);
-      for (int j = 0; j < n_other; ++j) load_other(0, j, row);
+      for (int j = 0; j < min(n_other, MT_RING); ++j) load_other(0, j, row);   // a half can need more boxes than the ring has
     }
   }
   if (warp == 1) {
@@ -515,7 +515,7 @@ mla_decode_tc_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_cons
           if (!ok) break;
           load_own(i, row);
         }
-        for (int j = 0; j < n_other && ok && i > 0; ++j) {
+        for (int j = i > 0 ? 0 : MT_RING; j < n_other && ok; ++j) {
           const int u = i * n_other + j;
           if (u >= MT_RING)
             ok = mbar_wait(b_emptyA + 8 * (u % MT_RING), (u / MT_RING - 1) & 1, abort_flag, p.status, EDL_TIMEOUT_PRODUCER);

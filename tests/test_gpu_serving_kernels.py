@@ -241,12 +241,14 @@ def test_decode_attention_with_more_sequences_than_sms(D, Dv, window, softcap):
 
 
 @pytest.mark.parametrize("H,L,R", [(17, 512, 64), (64, 512, 64), (128, 512, 64), (130, 512, 64), (40, 128, 64), (33, 320, 32),
-                                   (20, 72, 24), (18, 504, 72), (24, 256, 0), (5, 512, 64)])
+                                   (20, 72, 24), (18, 504, 72), (24, 256, 0), (5, 512, 64), (64, 320, 256),
+                                   (128, 384, 192), (96, 320, 136), (70, 384, 136), (64, 64, 512), (128, 128, 448), (64, 64, 384)])
 @pytest.mark.parametrize("lens", [[1], [64, 65, 0, 700, 129], [33] * 20 + [2000], [190] * 90])
 @pytest.mark.parametrize("window,splits", [(0, 1), (100, 1), (0, 3)])
 def test_latent_decode_many_heads(H, L, R, lens, window, splits):
     """Latent decode attention by either kernel: partial tiles, empty sequences, windows, every cluster size (by the number
-    of sequences), row widths that fill their last box or not, maxima that grow along a sequence, sinks."""
+    of sequences), row widths that fill their last box or not and that leave a half more score columns than its ring of
+    six boxes holds (seven or eight of them), maxima that grow along a sequence, sinks."""
     from easydel_b200.ops import _lib, serving as S
 
     torch.manual_seed(H + L)
