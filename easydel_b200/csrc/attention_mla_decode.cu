@@ -322,19 +322,23 @@ int launch_mla(const void* pages, long long num_pages, const MlaParams& p, cudaS
 // ---------------------------------------------------------------------------------------------------------------
 // tcgen05 form for many heads. With 16 heads per CTA every row was read from L2 eight times for 128 heads and multiplied
 // on mma.sync, two CTA-wide meetings per 32 rows. Here up to 128 heads are the M side of the products and a tile is 64
-// rows: S[heads, 64] = Q row^T (36 products for 576-wide rows), O[heads, 256] += P V (4 products). O takes 256 of the 512
+// rows: S[heads, 64] = Q row^T (36 products for 576-wide rows), O[heads, 256] += P V (8 products). O takes 256 of the 512
 // tensor-memory columns, so a CTA owns half of the (up to 512) value columns and computes the scores in full: 1.5 times the
 // multiplications of one pass, on a pipe that is otherwise idle, against rows that are read twice and not eight times.
-//   tensor memory: S / P even [0,64)  odd [64,128)   first 256 columns of Q, bf16 [128,256)   O [256,512)
+//   tensor memory: S / P (parts 32 columns apart) even [0,64)  odd [64,128)   first 256 columns of Q, bf16 [128,256)   O [256,512)
 //   shared memory: the other columns of Q (up to 5 boxes of 128 x 64), three stages of the half's up to 4 value boxes (64
 //   rows x 64 columns, held until PV), a ring of six boxes for the columns that only the scores need
 //   warp 0 loads rows; warp 1 issues S(i + 1) before PV(i), so that the softmax of tile i (warps 2..5, one thread per
-//   head) runs under the scores of tile i + 1; O is rescaled only when a maximum has grown by more than 2^8.
+//   head) runs under the scores of tile i + 1; O is rescaled only when a maximum has grown by more than 2^8. The largest
+//   probability is then no longer 1, exact in bf16, so P enters as two bf16 parts (16 bits): relative error against 64
+//   bits 1.66e-3, which is the rounding of the output, against 2.06e-3 with one part (32 sequences of 600 to 2000 rows)
+//   and 1.99e-3 of the mma.sync form. The second part costs 4.9 of 48 us; one part and a rescale for every new maximum
+//   46.2 us, but 2.07e-3 against 2.06e-3 of the mma.sync form on 100 sequences of 60 to 200 rows.
 // The keys of a sequence are cut over a cluster (1 to 4 CTAs, as many as fill the SMs). Each
 // sends every other one its part of that one's columns by one bulk copy between shared memories (4-byte loads from a
 // neighbour ran at 6 bytes a clock) and sums the parts in rank order.
-// 32 sequences of 600 to 2000 rows, 128 heads, 512 + 64 columns: 145 -> 43 us; one of 16000: 61 -> 27 us; 128 of 450 to
-// 1500: 393 -> 99 us. Bound now by the products with 64 rows (N = 64 takes as long as N = 128 would: 66 clocks).
+// 32 sequences of 600 to 2000 rows, 128 heads, 512 + 64 columns: 145 -> 48 us; one of 16000: 61 -> 29 us; 128 of 450 to
+// 1500: 393 -> 107 us. Bound now by the products with 64 rows (N = 64 takes as long as N = 128 would: 66 clocks).
 constexpr int MT_TK = 64;
 constexpr int MT_THREADS = 192;
 constexpr int MT_MAX_BOXES = 9;
@@ -567,8 +571,10 @@ mla_decode_tc_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_cons
 #pragma unroll
       for (int k = 0; k < MT_TK / 16; ++k)
         if (leader)
-          umma_f16_ts(tO, tmem + (i & 1) * 64 + k * 8, umma_smem_desc_sw128(vb + k * 2048, MT_BOX, 1024), id_o,
-                      (i | k) != 0 ? 1u : 0u);
+#pragma unroll
+          for (int part = 0; part < 2; ++part)
+            umma_f16_ts(tO, tmem + (i & 1) * 64 + part * 32 + k * 8, umma_smem_desc_sw128(vb + k * 2048, MT_BOX, 1024), id_o,
+                        (i | k | part) != 0 ? 1u : 0u);
       if (leader) {
         tc_commit(b_emptyV + 8 * (i % MT_STAGES));
         tc_commit(b_pv + 8 * (i & 1));
@@ -620,7 +626,7 @@ mla_decode_tc_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_cons
         }
         tc_wait_st();
       }
-      uint32_t pk[32];
+      uint32_t pk[32], pl[32];
       float ls[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
       for (int e = 0; e < 64; e += 2) {
@@ -628,9 +634,11 @@ mla_decode_tc_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_cons
         ls[e & 2] += e0;
         ls[(e & 2) + 1] += e1;
         pk[e >> 1] = pack_bf16x2(e0, e1);
+        pl[e >> 1] = pack_bf16x2(e0 - __uint_as_float(pk[e >> 1] << 16), e1 - __uint_as_float(pk[e >> 1] & 0xffff0000u));
       }
       l += (ls[0] + ls[1]) + (ls[2] + ls[3]);
       tmem_st_32x32b_x32(tmem + (i & 1) * 64 + row_sel, pk);
+      tmem_st_32x32b_x32(tmem + (i & 1) * 64 + 32 + row_sel, pl);
       tc_wait_st();
       tc_fence_before();
       mbar_arrive(b_p + 8 * (i & 1));

@@ -276,6 +276,25 @@ def test_latent_decode_many_heads(H, L, R, lens, window, splits):
         assert float((o[b].double() - want).abs().max()) <= tol, (b, n)
 
 
+@pytest.mark.parametrize("B,H,n", [(32, 128, 600), (4, 128, 2000), (100, 64, 300)])
+def test_latent_decode_of_peaked_scores_keeps_the_output_s_precision(B, H, n):
+    """Scores of a standard deviation of 2.25, so that a few keys carry most of a sum and maxima grow along a sequence: what is
+    left of the error against 64 bits is the rounding of the output to bf16 (7 stored bits: 2^-7 / sqrt(12) of a unit, over
+    mantissas that are log-uniform 0.7355 of that), and a tenth for the rest."""
+    from easydel_b200.ops import serving as S
+
+    torch.manual_seed(n)
+    per = (n + 127) // 128
+    pages = (torch.randn(B * per + 1, 128, 1, 576, device="cuda") * 1.5).to(torch.bfloat16)
+    table = (torch.randperm(B * per, device="cuda") + 1).view(B, per).to(torch.int32)
+    q = (torch.randn(B, H, 576, device="cuda") * 1.5).to(torch.bfloat16)
+    kv = torch.full((B,), n, dtype=torch.int32, device="cuda")
+    o = S.mla_decode_attention(q, pages, kv, table, scale=1 / 24)
+    rows = pages[table.long()].reshape(B, -1, 576)[:, :n].double()
+    want = torch.softmax(q.double() @ rows.mT / 24, -1) @ rows[..., :512]
+    assert float((o.double() - want).norm() / want.norm()) < 1.1 * 2.0 ** -7 / 12 ** 0.5 * 0.7355
+
+
 def _hash_u32(x):
     x &= 0xFFFFFFFF
     x = ((x ^ (x >> 16)) * 0x7FEB352D) & 0xFFFFFFFF
