@@ -28,6 +28,7 @@ __global__ void dequant_kernel(const uint8_t* __restrict__ codes, const __nv_bfl
   const int vecs = K / 8, groups = K / group;
   const bool wide = (ldo & 7) == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0;
   const bool small = (long long)N * vecs < (1LL << 32);
+  const bool pairs = (reinterpret_cast<uintptr_t>(codes) & 7) == 0;      // 8-bit codes may start on 4 bytes only
   for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < (long long)N * vecs;
        v += (long long)gridDim.x * blockDim.x) {
     const long long n = small ? (uint32_t)v / (uint32_t)vecs : v / vecs;
@@ -36,7 +37,8 @@ __global__ void dequant_kernel(const uint8_t* __restrict__ codes, const __nv_bfl
     if (BITS == 4) {
       w[0] = reinterpret_cast<const uint32_t*>(codes)[v];
     } else {
-      const uint2 t = reinterpret_cast<const uint2*>(codes)[v];
+      const uint32_t* at = reinterpret_cast<const uint32_t*>(codes) + 2 * v;
+      const uint2 t = pairs ? *reinterpret_cast<const uint2*>(at) : make_uint2(at[0], at[1]);
       w[0] = t.x, w[1] = t.y;
     }
     float f[8], sc = 0.f, zr = 0.f;
@@ -447,9 +449,14 @@ static int check_quant_args(const char* who, int bits, int N, int K, int group) 
   return 0;
 }
 
+// Codes start on 4 bytes or more.
 EDL_HOST_API int edl_dequant_bf16(const void* codes, const void* scales, const void* zeros, const float* lut, int bits,
                                   int N, int K, int group, void* out, long long ldo, void* stream) {
   if (check_quant_args("edl_dequant_bf16", bits, N, K, group)) return -1;
+  if ((uintptr_t)codes & 3) {
+    set_last_error("edl_dequant_bf16: codes must start on 4 bytes");
+    return -1;
+  }
   const long long total = (long long)N * (K / 8);
   long long blocks = (total + 255) / 256, cap = (long long)sm_count() * 16;
   if (blocks > cap) blocks = cap;

@@ -64,7 +64,8 @@ def test_products_at_the_limit_of_shared_memory(fmt, K, M):
 @pytest.mark.parametrize("odd", [False, True])
 def test_fused_product_at_its_edges(fmt, block, N, K, odd):
     """The fused product of a few rows: ragged weight rows and reductions, groups within, across and beyond a lane's 16 bytes
-    of codes, 1 to 16 activation rows; ``odd``: codes that start on 4 bytes only, strided activations, a bias."""
+    of codes, 1 to 16 activation rows, and the expansion behind more; ``odd``: codes that start on 4 bytes only, strided
+    activations, a bias."""
     from easydel_b200.layers.quantization import QuantizedTensor
 
     if block is not None and K % block:
@@ -85,8 +86,12 @@ def test_fused_product_at_its_edges(fmt, block, N, K, odd):
         # bf16 rounds the result by 2^-9; values keep 16 bits (2^-17 each), sums are fp32
         tol = 2.0 ** -8 * ref.abs() + 2.0 ** -16 * (x.double().abs() @ w.abs().t())
         assert ((y.double() - ref).abs() <= tol).all(), M
-    if not odd:
-        assert torch.equal(q.dequantize(), dequantize_reference(q).to(torch.bfloat16))
+    assert torch.equal(q.dequantize(), dequantize_reference(q).to(torch.bfloat16))
+    x = torch.randn(17, K, device="cuda").to(torch.bfloat16)
+    ref = x.double() @ w.t() + (0 if bias is None else bias.double())
+    # weights are rounded to bf16 as well: 2^-9 of each product
+    tol = 2.0 ** -8 * ref.abs() + 2.0 ** -9 * 1.01 * (x.double().abs() @ w.abs().t())
+    assert ((quantized_matmul(x, q, bias).double() - ref).abs() <= tol).all()
 
 
 @pytest.mark.gpu
