@@ -197,13 +197,15 @@ QGEMV_INPUTS = 47104     # inputs of 16 rows that its shared memory holds over a
 
 
 def quantized_matmul(x: torch.Tensor, q: QuantizedTensor, bias: torch.Tensor | None = None) -> torch.Tensor:
-    """``x @ W^T`` for a quantised ``W``; picks the fused GEMV for decode-sized inputs."""
+    """``x @ W^T`` for a quantised ``W``; picks the fused product, which has no backward pass, for decode-sized inputs that ask
+    for no gradient."""
     N, K = q.shape
     x2 = x.reshape(-1, K)
     M = x2.shape[0]
     per16 = 32 if q.bits == 4 else 16
     if x2.is_cuda and _lib.available() and x2.dtype == torch.bfloat16:
-        if M <= QGEMV_ROWS and q.group % per16 == 0 and K <= QGEMV_INPUTS * (2 if M <= 8 else 1):
+        graph = torch.is_grad_enabled() and (x.requires_grad or (bias is not None and bias.requires_grad))
+        if not graph and M <= QGEMV_ROWS and q.group % per16 == 0 and K <= QGEMV_INPUTS * (2 if M <= 8 else 1):
             if x2.stride(1) != 1 or x2.stride(0) % 8 or x2.data_ptr() % 16:
                 x2 = x2.clone(memory_format=torch.contiguous_format)
             out = torch.empty(M, N, dtype=torch.bfloat16, device=x.device)

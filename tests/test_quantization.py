@@ -95,6 +95,18 @@ def test_fused_product_at_its_edges(fmt, block, N, K, odd):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("M", [1, 8, 9, 16, 17])
+def test_gradients_pass_through_a_quantised_product_of_any_rows(M):
+    torch.manual_seed(M)
+    q = quantize(torch.randn(64, 256, device="cuda") * 0.05, "nf4")
+    x = torch.randn(M, 256, device="cuda").to(torch.bfloat16).requires_grad_()
+    dy = torch.randn(M, 64, device="cuda").to(torch.bfloat16)
+    (quantized_matmul(x, q).float() * dy).sum().backward()
+    want = dy.double() @ dequantize_reference(q).to(torch.bfloat16).double()
+    assert ((x.grad.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-5).all()      # one rounding to bf16
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("fmt", ["int8", "a4bit", "nf4", "mxfp4", "nvfp4", "mxfp8", "nvfp8"])
 @pytest.mark.parametrize("M", [1, 5, 8, 64])
 def test_cuda_kernels_match_reference(fmt, M):
