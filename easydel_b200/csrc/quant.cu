@@ -72,7 +72,9 @@ __global__ void dequant_kernel(const uint8_t* __restrict__ codes, const __nv_bfl
 //    transpose by shuffles), after which the word j of all four lies within bytes 16 j to 16 j + 15 of the block.
 //  * a 4-bit code byte holds two neighbouring k of one row: one 8-byte read of a table of 256 entries (16 copies, one per
 //    pair of banks) gives both values as bf16 pairs of their leading and of their remaining bits, which enter as two
-//    products, so that code books of fp32 values (nf4) keep 16 bits. Code books that are exact in bf16 skip the second.
+//    products, so that code books of fp32 values (nf4) keep 16 bits. Code books that are exact in bf16 skip the second. The
+//    error against 64 bits is that of fp32 code books on the FMA pipe to five digits (22016 x 4160, 1 row: 1.6579e-3 both,
+//    the output's rounding to bf16); a third part would cost a third more time (28672 x 4096, 4 rows: 44 -> 59 us).
 //    8-bit codes take one 4-byte read each for both parts.
 //  * activations are staged once per CTA in the order the fragments are read in (one 16-byte read per two steps).
 //  * a run (the part of a block in one group) is scaled into fp32 sums in the accumulator layout; zero points multiply the
@@ -89,6 +91,8 @@ constexpr int QG_MAX_M = 16;
 constexpr int QG_MAX_CLUSTER = 8;
 constexpr int QG_TABLE_BYTES = 256 * 128;
 constexpr int QG_SMEM_MAX = 216 * 1024;
+constexpr int QG_PASS_WARPS = 8;                            // of a CTA that takes row tiles in turn
+constexpr int QG_PASS_BYTES = 8 * 16 * QG_PASS_WARPS * 4;   // its sums of one pass
 
 struct QgParams {
   const __nv_bfloat16* x;
@@ -282,15 +286,17 @@ __device__ __forceinline__ void qg_rows(const QgParams& p, const unsigned char* 
   }
 }
 
-template <int BITS, int RUNS, int NT>
-__global__ void __launch_bounds__(NT == 1 ? 512 : 256, 1) qgemv_kernel(const QgParams p, const int cluster) {
+// PASSES: a CTA takes several row tiles in turn, with its table and activations in place (up to 25 more registers).
+template <int BITS, int RUNS, int NT, bool PASSES>
+__global__ void __launch_bounds__(NT == 1 ? 512 : 256, 1) qgemv_kernel(const QgParams p, const int cluster, const int passes,
+                                                                       const int x_bytes) {
   constexpr int BLOCK_K = 512 / BITS, PAIRS = BLOCK_K / 32;
   extern __shared__ __align__(128) unsigned char q_smem[];
   unsigned char* tab = q_smem;
   uint4* s_x = reinterpret_cast<uint4*>(q_smem + QG_TABLE_BYTES);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rows = blockDim.x / 2;                         // 16 per warp
-  const int tile = blockIdx.x / cluster, rank = blockIdx.x - tile * cluster;
+  const int first = blockIdx.x / cluster, rank = blockIdx.x - first * cluster;
   const int blocks = (p.K + BLOCK_K - 1) / BLOCK_K;
   const int blk0 = (int)((long long)blocks * rank / cluster), blk1 = (int)((long long)blocks * (rank + 1) / cluster);
 
@@ -336,43 +342,53 @@ __global__ void __launch_bounds__(NT == 1 ? 512 : 256, 1) qgemv_kernel(const QgP
   }
   __syncthreads();
 
-  float acc[NT][4];
+  // sums -> [activation row][weight row], then over the cluster in rank order
+  auto take_tile = [&](int tile, float* sums) {
+    float acc[NT][4];
 #pragma unroll
-  for (int n = 0; n < NT; ++n) acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.f;
-  const int row0 = tile * rows + warp * 16;
-  if (row0 < p.N) {
-    if (p.zeros) {
-      if (lo) qg_rows<BITS, RUNS, NT, true, true>(p, tab, s_x, row0, blk0, blk1, acc);
-      else qg_rows<BITS, RUNS, NT, false, true>(p, tab, s_x, row0, blk0, blk1, acc);
-    } else {
-      if (lo) qg_rows<BITS, RUNS, NT, true, false>(p, tab, s_x, row0, blk0, blk1, acc);
-      else qg_rows<BITS, RUNS, NT, false, false>(p, tab, s_x, row0, blk0, blk1, acc);
+    for (int n = 0; n < NT; ++n) acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.f;
+    const int row0 = tile * rows + warp * 16;
+    if (row0 < p.N) {
+      if (p.zeros) {
+        if (lo) qg_rows<BITS, RUNS, NT, true, true>(p, tab, s_x, row0, blk0, blk1, acc);
+        else qg_rows<BITS, RUNS, NT, false, true>(p, tab, s_x, row0, blk0, blk1, acc);
+      } else {
+        if (lo) qg_rows<BITS, RUNS, NT, true, false>(p, tab, s_x, row0, blk0, blk1, acc);
+        else qg_rows<BITS, RUNS, NT, false, false>(p, tab, s_x, row0, blk0, blk1, acc);
+      }
     }
-  }
-  // sums -> [activation row][weight row] over the table, then over the cluster in rank order
-  __syncthreads();
-  float* sums = reinterpret_cast<float*>(q_smem);
+    if (!PASSES) __syncthreads();                          // the sums go over the table
 #pragma unroll
-  for (int n = 0; n < NT; ++n)
+    for (int n = 0; n < NT; ++n)
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
-      sums[(n * 8 + (lane & 3) * 2 + (i & 1)) * rows + warp * 16 + (lane >> 2) + (i >> 1) * 8] = acc[n][i];
-  if (cluster > 1) cluster_sync_all();
-  else __syncthreads();
-  const uint32_t base = smem_u32(q_smem);
-  for (int v = rank * blockDim.x + threadIdx.x; v < p.M * rows; v += cluster * blockDim.x) {
-    const int m = v / rows, n = tile * rows + v % rows;
-    if (n >= p.N) continue;
-    float a = 0.f;
-    for (int r = 0; r < cluster; ++r) {
-      float t;
-      asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(t) : "r"(mapa_shared(base + v * 4, r)) : "memory");
-      a += t;
+      for (int i = 0; i < 4; ++i)
+        sums[(n * 8 + (lane & 3) * 2 + (i & 1)) * rows + warp * 16 + (lane >> 2) + (i >> 1) * 8] = acc[n][i];
+    if (cluster > 1) cluster_sync_all();
+    else __syncthreads();
+    const uint32_t base = smem_u32(sums);
+    for (int v = rank * blockDim.x + threadIdx.x; v < p.M * rows; v += cluster * blockDim.x) {
+      const int m = v / rows, n = tile * rows + v % rows;
+      if (n >= p.N) continue;
+      float a = 0.f;
+      for (int r = 0; r < cluster; ++r) {
+        float t;
+        asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(t) : "r"(mapa_shared(base + v * 4, r)) : "memory");
+        a += t;
+      }
+      if (p.bias) a += __bfloat162float(p.bias[n]);
+      p.out[m * p.ldo + n] = __float2bfloat16(a);
     }
-    if (p.bias) a += __bfloat162float(p.bias[n]);
-    p.out[m * p.ldo + n] = __float2bfloat16(a);
+    __syncwarp();
+  };
+  if constexpr (PASSES) {
+    // two buffers in turn behind the activations, one meeting per pass: a buffer is written again behind the next meeting,
+    // which everybody reaches after reading it
+    float* const buffers = reinterpret_cast<float*>(q_smem + QG_TABLE_BYTES + x_bytes);
+    const int clusters = gridDim.x / cluster;
+    for (int pass = 0; pass < passes; ++pass) take_tile(first + pass * clusters, buffers + (pass & 1) * (NT * 8 * rows));
+  } else {
+    take_tile(first, reinterpret_cast<float*>(q_smem));
   }
-  __syncwarp();
   if (cluster > 1) cluster_sync_all();   // no CTA leaves while another may still read its sums
 }
 
@@ -385,38 +401,61 @@ int launch_qgemv(const QgParams& p, cudaStream_t stream) {
   // a CTA's start 6000, and clusters of 4 or 8 leave the SMs of a GPC that do not make up another one idle (132 and 128 of
   // 148 take part). One B200, nf4, 4 rows, us for (warps, parts): 6144 x 4096 (12, 4) 14.7, (16, 4) 16.4, (8, 2) 19.6, (8, 8)
   // 21.8, (8, 1) 32.3; 4096 x 14336 (8, 8) 25.2, (8, 4) 30.7; 28672 x 4096 (13, 1) 44.2, (13, 2) 50.2, (8, 4) 58.6.
-  int warps = 0, cluster = 0;
-  long long best = 0;
+  // Five warps put two of them on one of the four schedulers (22016 x 4096, two CTAs of five per SM 40, one of ten 36); with
+  // 16 rows, whose products take longer, that shows where the registers hold one such CTA only (mxfp4 28672 x 4096 99, 64).
+  int warps = 0, cluster = 0, passes = 1;
+  long long best = 0, smem = 0, grid = 0;
   for (int c = 1; c <= QG_MAX_CLUSTER && c <= blocks; c *= 2) {
     if (smem_of(c) > QG_SMEM_MAX) continue;
     const int usable = c == 8 ? sms * 128 / 148 : c == 4 ? sms * 132 / 148 : c == 2 ? sms & ~1 : sms;
     for (int w = 4; w <= (NT == 1 ? 16 : 8); ++w) {
-      const long long ctas = (long long)((row_tiles + w - 1) / w) * c, per_sm = (ctas + usable - 1) / usable;
+      if (w == 5 && (NT == 1 || RUNS == 4)) continue;
+      const long long tiles = (row_tiles + w - 1) / w, per_sm = (tiles * c + usable - 1) / usable;
       const int by_smem = (int)(QG_SMEM_MAX / smem_of(c)), by_regs = (NT == 1 ? 16 : RUNS == 4 ? 10 : 12) / w;
       const int most = by_smem < by_regs ? by_smem : by_regs, resident = (int)(per_sm < most ? per_sm : most);
-      const long long cost = (per_sm + resident - 1) / resident * ((1100 + 70LL * resident * w) * ((blocks + c - 1) / c) + 6000);
-      if (!warps || cost < best) best = cost, warps = w, cluster = c;
+      const long long rounds = (per_sm + resident - 1) / resident;
+      const long long cost = rounds * ((1100 + 70LL * resident * w) * ((blocks + c - 1) / c) + 6000);
+      if (!warps || cost < best) best = cost, warps = w, cluster = c, smem = smem_of(c), grid = tiles * c, passes = (int)rounds;
     }
+  }
+  // Where that takes several rounds of CTAs, two CTAs of eight warps stay on every SM instead and take row tiles in turn: their
+  // start is paid once, and half the reduction per tile fills the last pass better. Up to 8 rows (more need the registers);
+  // us, in rounds / in passes, 1 row: nf4 55296 x 5120 88.1 / 80.0, 57344 x 8192 153.2 / 144.6, 128256 x 4096 171 / 148.
+  // Two CTAs interleave better than the clocks above say, unless zero points or 8-bit codes load them more: 57344 x 8192 int8
+  // 168 / 193, 4-bit with zero points 136 / 147, and those stay in rounds by this.
+  const bool rounds = passes > 1;
+  const int part = BITS == 4 && !p.zeros ? 9 : 10;
+  passes = 1;
+  for (int c = 1; NT == 1 && rounds && c <= 2 && c <= blocks; c *= 2) {
+    const long long need = smem_of(c) + 2 * QG_PASS_BYTES;
+    if (need > QG_SMEM_MAX) continue;
+    const long long tiles = (row_tiles + QG_PASS_WARPS - 1) / QG_PASS_WARPS, here = sms / c * (2 * need <= QG_SMEM_MAX ? 2 : 1);
+    const long long turns = (tiles + here - 1) / here, on_sm = 2 * need <= QG_SMEM_MAX ? 2 * QG_PASS_WARPS : QG_PASS_WARPS;
+    if (turns < 2) continue;
+    const long long cost = turns * ((1100 + 70 * on_sm) * part * ((blocks + c - 1) / c) / 10 + (c > 1 ? 1500 : 500)) + 6000;
+    if (cost < best) best = cost, warps = QG_PASS_WARPS, cluster = c, smem = need, grid = here * c, passes = (int)turns;
   }
   if (!warps) {
     set_last_error("edl_qgemv: %d activation rows of %d do not fit into shared memory", p.M, p.K);
     return -1;
   }
-  auto kern = qgemv_kernel<BITS, RUNS, NT>;
-  static bool attr_set[64] = {false};
+  auto kern = qgemv_kernel<BITS, RUNS, NT, false>;
+  if constexpr (NT == 1)
+    if (passes > 1) kern = qgemv_kernel<BITS, RUNS, NT, true>;
+  static bool attr_set[64][2] = {};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64) dev = 0;
-  if (!attr_set[dev]) {
+  if (!attr_set[dev][passes > 1]) {
     if (check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, QG_SMEM_MAX),
                    "cudaFuncSetAttribute(qgemv)"))
       return -1;
-    attr_set[dev] = true;
+    attr_set[dev][passes > 1] = true;
   }
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)((row_tiles + warps - 1) / warps * cluster), 1, 1);
+  cfg.gridDim = dim3((unsigned)grid, 1, 1);
   cfg.blockDim = dim3(warps * 32, 1, 1);
-  cfg.dynamicSmemBytes = (size_t)smem_of(cluster);
+  cfg.dynamicSmemBytes = (size_t)smem;
   cfg.stream = stream;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeClusterDimension;
@@ -425,7 +464,7 @@ int launch_qgemv(const QgParams& p, cudaStream_t stream) {
   at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  return check_cuda(cudaLaunchKernelEx(&cfg, kern, p, cluster), "qgemv launch");
+  return check_cuda(cudaLaunchKernelEx(&cfg, kern, p, cluster, passes, (int)(smem_of(cluster) - QG_TABLE_BYTES)), "qgemv launch");
 }
 
 template <int BITS, int RUNS>

@@ -95,6 +95,22 @@ def test_fused_product_at_its_edges(fmt, block, N, K, odd):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("fmt,block", [("nf4", 64), ("a4bit", 32), ("mxfp4", None), ("int8", 128), ("a8bit", 64)])
+@pytest.mark.parametrize("N,K", [(60003, 256), (45000, 1152), (38000, 3584)])
+def test_fused_product_of_more_rows_than_a_round(fmt, block, N, K):
+    """Weight rows beyond what all SMs take at once: CTAs that go over several row tiles, the last ones past the end."""
+    torch.manual_seed(N)
+    q = quantize(torch.randn(N, K, device="cuda") * 0.05, EasyDeLQuantizationConfig(fmt, block_size=block))
+    w = dequantize_reference(q)
+    for M in (1, 5, 8):
+        x = torch.randn(M, K, device="cuda").to(torch.bfloat16)
+        bias = torch.randn(N, device="cuda", dtype=torch.bfloat16)
+        ref = x.double() @ w.double().t() + bias.double()
+        tol = 2.0 ** -8 * ref.abs() + 2.0 ** -16 * (x.double().abs() @ w.double().abs().t())     # as above
+        assert ((quantized_matmul(x, q, bias).double() - ref).abs() <= tol).all(), M
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("M", [1, 8, 9, 16, 17])
 def test_gradients_pass_through_a_quantised_product_of_any_rows(M):
     torch.manual_seed(M)
