@@ -25,11 +25,11 @@
 //     and chunk for the delta rule with DK = 128, 102 for the state space, at about 20 clocks each, and with one warp per
 //     scheduler the chain y -> T -> P behind them.
 //
-// 5328 + 2864 tokens, 32 heads of 128 x 128: 0.73 ms (eight tokens at a time on the FMA pipe 1.90 ms, one at a time 19.4 ms);
-// 6000 tokens in three sequences, 64 state-space heads of 64 x 128: 0.32 ms (0.74 ms, 4.4 ms). Bytes at the copy rate: 43 and
+// 5328 + 2864 tokens, 32 heads of 128 x 128: 0.64 ms (eight tokens at a time on the FMA pipe 1.90 ms, one at a time 19.4 ms);
+// 6000 tokens in three sequences, 64 state-space heads of 64 x 128: 0.30 ms (0.74 ms, 4.4 ms). Bytes at the copy rate: 43 and
 // 18 us. State-space sequences are cut into segments where that fills the GPU (cs_span): 8192 tokens of one sequence, 64 heads
-// 0.93 -> 0.38 ms, 8 heads 0.91 -> 0.09 ms. A value that is not finite spoils its column for the whole chunk (a zero weight
-// times infinity), not only from its token on.
+// 0.93 -> 0.38 ms, 8 heads 0.91 -> 0.09 ms. A value that is not finite reaches its column from its token on only, as in
+// a walk token by token: a chunk that holds one is summed on the FMA pipe (cs_triangle).
 // Compiled without fast-math.
 #include "common.cuh"
 
@@ -142,6 +142,61 @@ __device__ __forceinline__ void cs_split_block(const float (&c0)[4], const float
   cs_split(c0[2], c0[3], a[0][1], a[1][1], a[2][1]);
   cs_split(c1[0], c1[1], a[0][2], a[1][2], a[2][2]);
   cs_split(c1[2], c1[3], a[0][3], a[1][3], a[2][3]);
+}
+
+// Values that a product with zero does not take out: not finite, or so large that a bf16 part is not.
+__device__ __forceinline__ bool cs_unsafe(const float (&r)[2][4]) {
+  bool x = false;
+#pragma unroll
+  for (int j = 0; j < 2; ++j)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) x |= !(fabsf(r[j][e]) < 3.38e38f);
+  return __any_sync(0xffffffffu, x);
+}
+
+// sum_{i <= j} W_ji r_i for the tokens j of this lane, token by token, so that what is not finite reaches no token before its
+// own (the products multiply it with the zeros above W's diagonal). W as stored: parts in the order of a right operand; r: the
+// first N parts of a left operand.
+template <int N>
+__device__ __forceinline__ void cs_triangle(const uint8_t* parts, const uint32_t (&a)[3][4], int lane, float (&out)[2][4]) {
+  const int quad = lane & 3;
+  float r[2][4];
+#pragma unroll
+  for (int j = 0; j < 2; ++j)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      auto part = [&](int n) { const uint32_t w = a[n][2 * j + (e >> 1)]; return __uint_as_float(e & 1 ? w & 0xffff0000u : w << 16); };
+      r[j][e] = part(0);
+      if (N > 1 && isfinite(r[j][e])) r[j][e] += part(1) + part(2);
+    }
+#pragma unroll
+  for (int j = 0; j < 2; ++j)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) out[j][e] = 0.f;
+#pragma unroll 1
+  for (int i = 0; i < CS_C; ++i) {
+    const int from = (lane & 28) + ((i & 7) >> 1);
+    float v[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const float x = i & 1 ? r[0][2 * h + 1] : r[0][2 * h], y = i & 1 ? r[1][2 * h + 1] : r[1][2 * h];
+      v[h] = __shfl_sync(0xffffffffu, i & 8 ? y : x, from);
+    }
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int t = 2 * quad + e;
+        const uint8_t* at = parts + (t * 4 + ((i & 7) >> 1)) * 16 + (2 * j + (i >> 3)) * 4 + (i & 1) * 2;
+        float w = 0.f;
+#pragma unroll
+        for (int part = 2; part >= 0; --part) w += __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(at + part * 512));
+        if (8 * j + t >= i) {
+          out[j][e] = fmaf(w, v[0], out[j][e]);
+          out[j][e + 2] = fmaf(w, v[1], out[j][e + 2]);
+        }
+      }
+  }
 }
 
 // ---- coefficients -----------------------------------------------------------------------------------------------------
@@ -417,6 +472,7 @@ __global__ void __launch_bounds__(CS_THREADS) chunk_scan_kernel(const CsParams p
           r[j][e] = beta[t] * r[j][e] - eb[t] * (yk[0][j][e] + yk[1][j][e]);
         }
       cs_split_block(r[0], r[1], ra);
+      const bool unsafe = cs_unsafe(r);
       uint4 tp[3];
 #pragma unroll
       for (int i = 0; i < 3; ++i) tp[i] = *reinterpret_cast<const uint4*>(rec + CS_T + i * 512 + lane * 16);
@@ -437,11 +493,13 @@ __global__ void __launch_bounds__(CS_THREADS) chunk_scan_kernel(const CsParams p
 #pragma unroll
         for (int e = 0; e < 4; ++e) r[j][e] = lead[j][e] + rest[j][e];
       }
+      if (unsafe) cs_triangle<3>(rec + CS_T, ra, lane, r);
       cs_split_block(r[0], r[1], ra);
     } else {                            // the inputs are exact in one part
 #pragma unroll
       for (int i = 0; i < 4; ++i) ra[0][i] = vf[i];
     }
+    const bool unsafe = !LOCAL && cs_unsafe(r);
     // ---- the state behind the chunk
     {
       const float* tail = reinterpret_cast<const float*>(rec + CS_TAIL);
@@ -477,6 +535,7 @@ __global__ void __launch_bounds__(CS_THREADS) chunk_scan_kernel(const CsParams p
 #pragma unroll
       for (int i = 0; i < 3; ++i) tp[i] = *reinterpret_cast<const uint4*>(rec + CS_P + i * 512 + lane * 16);
       const int n = min(CS_C, t1 - tb);
+      float x[2][4];                    // what the chunk's own tokens give
 #pragma unroll
       for (int j = 0; j < 2; ++j) {
         float lead[4] = {0.f, 0.f, 0.f, 0.f}, rest[4] = {0.f, 0.f, 0.f, 0.f};
@@ -491,14 +550,19 @@ __global__ void __launch_bounds__(CS_THREADS) chunk_scan_kernel(const CsParams p
           cs_mma(rest, ra[0], EDL_B(1));
         }
         cs_mma(lead, ra[0], EDL_B(0));
+#pragma unroll
+        for (int e = 0; e < 4; ++e) x[j][e] = lead[e] + rest[e];
+      }
+      if (unsafe) cs_triangle<MODE == CS_DELTA ? 3 : 1>(rec + CS_P, ra, lane, x);
 #undef EDL_B
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
           const int t = 8 * j + 2 * quad + (e & 1), c = col + 8 * (e >> 1);
-          const float o = es[t] * (yq[0][j][e] + yq[1][j][e]) + (lead[e] + rest[e]);
+          const float o = es[t] * (yq[0][j][e] + yq[1][j][e]) + x[j][e];
           if (t < n && c < DV) p.o[((long long)(tb + t) * H + h) * DV + c] = __float2bfloat16(o);
         }
-      }
     }
     st = st == CS_STAGES - 1 ? 0 : st + 1;
   }

@@ -79,6 +79,36 @@ def test_delta_rule_cuda(DK, DV, kda):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("what", [float("inf"), -float("inf"), float("nan"), 3.3895e38])
+@pytest.mark.parametrize("at", [0, 7, 18, 31, 40])
+def test_scans_keep_what_is_not_finite_from_earlier_tokens(what, at):
+    """A value that is not finite (or is once it has been multiplied) reaches its head's column from its token on and nothing
+    else: not the tokens before it, that share products of sixteen with it, nor other columns, heads or sequences. A key that
+    is not finite does so for all columns of its head."""
+    torch.manual_seed(5)
+    dev, T, H, D = "cuda", 90, 2, 64
+    cu = torch.tensor([0, 45, 90], dtype=torch.int32, device=dev)
+    rnd = lambda *s: torch.randn(*s, device=dev)
+    q, k = (torch.nn.functional.normalize(rnd(T, H, D), dim=-1).to(torch.bfloat16) for _ in range(2))
+    v, g, beta = rnd(T, H, D).to(torch.bfloat16), -torch.rand(T, H, device=dev), torch.rand(T, H, device=dev).to(torch.bfloat16)
+    B, C = rnd(T, 1, D).to(torch.bfloat16), rnd(T, 1, D).to(torch.bfloat16)
+    dt, A, Dv = rnd(T, H).to(torch.bfloat16), -torch.rand(H, device=dev) - 0.5, torch.randn(H, device=dev)
+    ops = [(lambda v, k: ssm.gated_delta_rule(q, k, v, g, beta, None, cu), k), (lambda v, k: ssm.gated_delta_rule(
+               q, k, v, g[..., None].expand(T, H, D), beta, None, cu), k), (lambda v, B: ssm.ssd_scan(v, dt, A, B, C, Dv, None, True, cu), B)]
+    for op, key in ops:
+        clean = op(v, key).float()
+        v2, k2 = v.clone(), key.clone()
+        v2[at, 1, 5] = what
+        k2[at, -1] = float("nan")
+        for got, hit in ((op(v2, key), (slice(at, 45), 1, 5)), (op(v, k2), (slice(at, 45), slice(1 if key is k else 0, 2)))):
+            off = torch.zeros(T, H, D, dtype=torch.bool, device=dev)
+            off[hit] = True
+            assert _close(got.float()[~off], clean[~off])
+            if what != 3.3895e38:
+                assert not got[hit][1:].isfinite().any()
+
+
+@pytest.mark.gpu
 def test_ragged_conv1d_cuda():
     torch.manual_seed(4)
     dev, T, Cn, W = "cuda", 50, 96, 4
