@@ -4,9 +4,8 @@ from __future__ import annotations
 
 import torch
 from torch import nn
-from torch.nn.modules.module import _global_forward_hooks
 
-from ..ops import functional as F, stream
+from ..ops import functional as F, remat, stream
 from ..ops.reference import ACT2FN
 from .linears import ColumnParallelLinear, RowParallelLinear
 
@@ -35,7 +34,8 @@ class GatedMLP(nn.Module):
         """Whether :meth:`forward` returns what ``down_proj`` computes, with nothing in between that could read it."""
         d = self.down_proj
         return (type(self) is GatedMLP and type(d) is RowParallelLinear and d.tp_size == 1 and d.scale is None
-                and self.down_multiplier == 1.0 and not (self._forward_hooks or d._forward_hooks or _global_forward_hooks))
+                and self.down_multiplier == 1.0 and remat.runs_as_defined(self, _GATED_FORWARD)
+                and remat.runs_as_defined(d, _ROW_FORWARD))
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         gu = self.gate_up_proj(x)
@@ -51,6 +51,9 @@ class GatedMLP(nn.Module):
             raise NotImplementedError("fp32-stream feed-forwards: no multipliers, no bias on the way down")
         gu = stream.linear(h, self.gate_up_proj.weight, self.gate_up_proj.bias)
         return stream.branch_product(stream.gated_unit(gu, self.act), self.down_proj.weight, base)
+
+
+_GATED_FORWARD, _ROW_FORWARD = GatedMLP.forward, RowParallelLinear.forward      # before anybody puts others in their place
 
 
 class PlainMLP(nn.Module):

@@ -513,8 +513,8 @@ class DecoderLayer(nn.Module):
                 h, x = self.input_layernorm.forward_with_residual(pending, x)
             a = self._mix(h, positions, segment_ids, cache_view, attn_meta)
             h, x = self.post_attention_layernorm.forward_with_residual(a, x)
-            with remat.returned_as_is(type(self).forward is DecoderLayer.forward and not self._forward_hooks
-                                      and type(self.mlp) is GatedMLP and self.mlp.ends_in_product()):
+            with remat.returned_as_is(remat.runs_as_defined(self, _LAYER_FORWARD) and type(self.mlp) is GatedMLP
+                                      and self.mlp.ends_in_product()):
                 m = self.mlp(h)
             if self.is_moe:
                 m, rl = m
@@ -549,6 +549,9 @@ class DecoderLayer(nn.Module):
         if spec.sandwich_norm:
             m = self.post_feedforward_layernorm(m)
         return x + m * rm, None, rl
+
+
+_LAYER_FORWARD = DecoderLayer.forward        # before anybody puts another one in its place
 
 
 class DecoderModel(EasyDeLBaseModule):
@@ -645,7 +648,8 @@ class DecoderModel(EasyDeLBaseModule):
         if policy and self.training and torch.is_grad_enabled() and cache_view is None:
             # recompute unit under the configured save policy (full recompute, saved dots, saved names ...)
             return remat.recompute_unit(lambda a, b, c, d: layer(a, b, c, d, None, None), self.remat_policy(),
-                                        (x, _resolve(pending), positions, segment_ids), whole_layer=True)
+                                        (x, _resolve(pending), positions, segment_ids),
+                                        whole_layer=remat.runs_as_defined(layer, _LAYER_FORWARD))
         return layer(x, pending, positions, segment_ids, cache_view, attn_meta)
 
     def forward(self, input_ids: torch.Tensor | None = None, attention_mask: torch.Tensor | None = None,

@@ -21,6 +21,7 @@ import threading
 import typing as tp
 
 import torch
+from torch.nn.modules.module import _global_forward_hooks
 
 _ALIASES = {
     "attn_qkv": ("attn_qkv", "attn_query", "attn_key", "attn_value"),
@@ -115,6 +116,13 @@ def keep_output(name: str | None, kind: str, value) -> None:
     t = _tape
     if t.mode == "record" and t.policy.saves(name, kind):
         t.store.append(value)
+
+
+def runs_as_defined(module, forward) -> bool:
+    """Whether calling ``module`` is calling ``forward``, the function its class was defined with, and nothing else sees what
+    comes out: neither the class nor the instance has got another one, and there is no forward hook."""
+    return (type(module).forward is forward and "forward" not in vars(module)
+            and not (module._forward_hooks or _global_forward_hooks))
 
 
 class returned_as_is:

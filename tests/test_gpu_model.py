@@ -178,3 +178,51 @@ def test_recompute_leaves_out_only_what_nobody_reads(span):
         got.append([y.detach(), p.detach(), x.grad] + [w.grad for w in list(a.parameters()) + list(b.parameters())])
     for u, v in zip(*got):
         assert torch.equal(u, v)
+
+
+@pytest.mark.parametrize("where", ["product", "feed-forward", "class", "layer", "layer around it"])
+def test_recompute_of_wrapped_forwards_reads_real_values(where, monkeypatch):
+    """A forward that somebody put in the place of a layer's, its feed-forward's or their last product's reads what that
+    returns, in the recompute too: the gradient of a scale learnt there equals the one without recomputation."""
+    from easydel_b200.layers.mlp import GatedMLP
+    from easydel_b200.modules.llama import LlamaConfig, LlamaForCausalLM
+
+    got = []
+    for policy in ("", "nothing_saveable"):
+        cfg = LlamaConfig(vocab_size=256, hidden_size=256, intermediate_size=512, num_hidden_layers=2, num_attention_heads=4,
+                          num_key_value_heads=2, head_dim=64, max_position_embeddings=256, gradient_checkpointing=policy)
+        model = LlamaForCausalLM.sequential_init(cfg, dtype=torch.bfloat16, param_dtype=torch.bfloat16, device="cuda", seed=3).train()
+        scale = torch.nn.Parameter(torch.tensor(1.25, device="cuda", dtype=torch.bfloat16))
+        layer = model.model.layers[0]
+
+        def scaled(f):
+            def g(*args, **kw):
+                out = f(*args, **kw)
+                return (out[0], out[1] * scale, out[2]) if isinstance(out, tuple) else out * scale
+            return g
+
+        with monkeypatch.context() as mp:
+            if where == "class":
+                mp.setattr(GatedMLP, "forward", scaled(GatedMLP.forward))
+            elif where == "layer around it":
+                class Around(torch.nn.Module):
+                    def __init__(self, inner):
+                        super().__init__()
+                        self.inner = inner
+                        self.call = scaled(inner)
+
+                    def forward(self, *args):
+                        return self.call(*args)
+
+                model.model.layers[0] = Around(layer)
+            else:
+                m = {"product": layer.mlp.down_proj, "feed-forward": layer.mlp, "layer": layer}[where]
+                m.forward = scaled(m.forward)
+            ids = torch.arange(200, device="cuda")[None] % 256
+            junk = torch.full((64, 200, 256), 1e4, device="cuda", dtype=torch.bfloat16)      # what empty buffers then hold
+            del junk
+            h = model.model(input_ids=ids).last_hidden_state
+            h.float().square().sum().backward()
+        got.append([scale.grad] + [p.grad for p in layer.parameters()])
+    for u, v in zip(*got):
+        assert torch.equal(u, v)
