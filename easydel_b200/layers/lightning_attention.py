@@ -57,9 +57,9 @@ class LightningAttention(nn.Module):
         qkv = self.act(self.lqkv(hidden)).view(B * T, self.h, 3 * self.d)
         q, k, v = torch.split(qkv, self.d, dim=-1)
         if segment_ids is not None and state is None:
-            from ..ops.attention import segment_ids_to_cu_seqlens
+            from ..ops.attention import segment_plan
 
-            cu, _ = segment_ids_to_cu_seqlens(segment_ids)
+            cu, _ = segment_plan(segment_ids)
         else:
             cu = getattr(state, "cu", None)       # a serving state names its own (ragged) sequence bounds
             if cu is None:

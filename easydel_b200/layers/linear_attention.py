@@ -88,9 +88,9 @@ class GatedDeltaNet(nn.Module):
             b, a = self.in_proj_b(hidden), self.in_proj_a(hidden)
         mixed = torch.cat([q, k, v], -1).reshape(B * T, self.conv_dim)
         if segment_ids is not None and state is None:
-            from ..ops.attention import segment_ids_to_cu_seqlens
+            from ..ops.attention import segment_plan
 
-            cu, _ = segment_ids_to_cu_seqlens(segment_ids)
+            cu, _ = segment_plan(segment_ids)
         else:
             cu = getattr(state, "cu", None)       # a serving state names its own (ragged) sequence bounds
             if cu is None:
@@ -160,9 +160,9 @@ class KimiDeltaAttention(nn.Module):
     def forward(self, hidden, segment_ids=None, state: KDAState | None = None):
         B, T, _ = hidden.shape
         if segment_ids is not None and state is None:
-            from ..ops.attention import segment_ids_to_cu_seqlens
+            from ..ops.attention import segment_plan
 
-            cu, _ = segment_ids_to_cu_seqlens(segment_ids)
+            cu, _ = segment_plan(segment_ids)
         else:
             cu = getattr(state, "cu", None)       # a serving state names its own (ragged) sequence bounds
             if cu is None:

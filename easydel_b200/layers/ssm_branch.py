@@ -74,9 +74,9 @@ class SSDMixer(nn.Module):
         proj = self.in_proj(h * self.in_multiplier) * self.mup_vector.to(h.dtype)
         z, xbc, dt = proj[..., :I], proj[..., I:I + self.conv_dim], proj[..., I + self.conv_dim:]
         if segment_ids is not None and state is None:
-            from ..ops.attention import segment_ids_to_cu_seqlens
+            from ..ops.attention import segment_plan
 
-            cu, _ = segment_ids_to_cu_seqlens(segment_ids)
+            cu, _ = segment_plan(segment_ids)
         else:
             cu = getattr(state, "cu", None)       # a serving state names its own (ragged) sequence bounds
             if cu is None:

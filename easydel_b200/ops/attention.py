@@ -145,19 +145,29 @@ def segment_ids_to_cu_seqlens(segment_ids: torch.Tensor):
 
 
 def with_segment_plan(segment_ids: torch.Tensor) -> torch.Tensor:
-    """The same segment ids for the layers of one forward pass, as a tensor of its own that carries its varlen metadata (which
-    needs the host to wait for the device): found once per pass, not once per layer and recomputation."""
+    """The same segment ids for the layers of one forward pass, as a tensor of its own that keeps its varlen metadata (which
+    needs the host to wait for the device): found by the first layer that asks (:func:`segment_plan`), not once per layer and
+    recomputation, and not at all where no layer does."""
     own = segment_ids.view(segment_ids.shape)
-    own.varlen_plan = segment_ids_to_cu_seqlens(segment_ids)
+    own.varlen_plan = []
     return own
+
+
+def segment_plan(segment_ids: torch.Tensor):
+    """:func:`segment_ids_to_cu_seqlens`, once per forward pass for ids from :func:`with_segment_plan`."""
+    plan = getattr(segment_ids, "varlen_plan", None)
+    if plan is None:
+        return segment_ids_to_cu_seqlens(segment_ids)
+    if not plan:
+        plan.append(segment_ids_to_cu_seqlens(segment_ids))
+    return plan[0]
 
 
 def flash_attention(q, k, v, *, causal=True, scale=None, segment_ids=None, sliding_window=None, softcap=0.0,
                     sinks=None, cu_seqlens=None, max_seqlen=None):
     """Differentiable attention. ``[B,T,H,D]`` inputs; ``segment_ids`` or ``cu_seqlens`` select packed-document masking."""
     if segment_ids is not None and cu_seqlens is None:
-        plan = getattr(segment_ids, "varlen_plan", None)
-        cu_seqlens, max_seqlen = plan if plan is not None else segment_ids_to_cu_seqlens(segment_ids)
+        cu_seqlens, max_seqlen = segment_plan(segment_ids)
     if cu_seqlens is not None:
         if max_seqlen is None:
             max_seqlen = int((cu_seqlens[1:] - cu_seqlens[:-1]).max().item())

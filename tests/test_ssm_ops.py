@@ -341,3 +341,31 @@ def test_ssd_segments_match_the_tokens_one_by_one(lens, H, P, G, N, seg, with_st
     if with_state:
         assert (s1 - s2).abs().max() < 1e-5 * s2.abs().max()
     assert ((got.float() - want).abs() <= 2 ** -8 * want.abs() + 1e-5 * want.abs().max()).all()
+
+
+def test_layers_of_a_packed_pass_share_its_segment_plan(monkeypatch):
+    """The bounds of packed documents make the host wait for the device: the first layer that asks finds them, the others (and
+    recomputations) take what it found, and a pass whose layers do not ask finds none. Without a plan, as before, each its own."""
+    from easydel_b200.layers.lightning_attention import LightningAttention
+    from easydel_b200.layers.linear_attention import GatedDeltaNet, KimiDeltaAttention
+    from easydel_b200.layers.ssm_branch import SSDMixer
+    from easydel_b200.ops import attention
+
+    torch.manual_seed(7)
+    found = []
+    real = attention.segment_ids_to_cu_seqlens
+    monkeypatch.setattr(attention, "segment_ids_to_cu_seqlens", lambda ids: found.append(1) or real(ids))
+    layers = [LightningAttention(32, 2, 16, 2), GatedDeltaNet(32, 2, 2, 16, 16), KimiDeltaAttention(32, 2, 16, 16, gate_low_rank_dim=8),
+              SSDMixer(32, 32, 2, 16, 1, 16)]
+    x = torch.randn(2, 12, 32)
+    ids = torch.tensor([[1] * 5 + [2] * 7, [1] * 12])
+    with torch.no_grad():
+        want = [l(x, segment_ids=ids) for l in layers]
+        assert len(found) == len(layers)
+        found.clear()
+        own = attention.with_segment_plan(ids)
+        assert not found
+        got = [l(x, segment_ids=own) for l in layers] + [layers[0](x, segment_ids=own)]
+    assert len(found) == 1
+    for a, b in zip(got, want + want[:1]):
+        assert torch.equal(a, b)
