@@ -65,6 +65,9 @@ struct CsParams {
   float* state;                      // delta [B, H, DK, DV], state space [B, H, DV, DK]; or null
   __nv_bfloat16* o;                  // [T, H, DV]
   bool vec_v;                        // values can be fetched 16 bytes at a time
+  int w0, w1;                        // the window of tokens this launch takes
+  const float* carry_in;             // without `state`: what the sequence cut by the window's start left in front of it, and
+  float* carry_out;                  // where the one cut by its end leaves its own, [H, state]
   int seg;                           // tokens of a segment (a multiple of 16), or 0: sequences are walked from end to end
   float *seg_state, *seg_decay;      // [segments, H, DV, DK], [segments, H]
 };
@@ -73,6 +76,10 @@ struct CsParams {
 // plus what its tokens leave in an empty state. A first pass computes the latter (48 of the 102 products of a chunk), one
 // thread per element carries states from segment to segment, then every segment runs in full from the state in front of it.
 // A segment's place, as a chunk's: unique and increasing, below T / seg + B + 1.
+// Long inputs go in windows of tokens, so that the records of one fit a workspace of bounded size: a window's part of every
+// sequence is a sequence of its own whose state comes from the one before.
+__device__ __forceinline__ int cs_pos(const CsParams& p, int b) { return min(max(p.cu[b], p.w0), p.w1); }
+
 struct CsSpan {
   int b, t0, t1, slot;
 };
@@ -81,26 +88,36 @@ __device__ __forceinline__ CsSpan cs_span(const CsParams& p, int z) {
   s.slot = z;
   if (p.seg == 0) {
     s.b = z;
-    s.t0 = p.cu[z];
-    s.t1 = p.cu[z + 1];
+    s.t0 = cs_pos(p, z);
+    s.t1 = cs_pos(p, z + 1);
     return s;
   }
   int lo = 0, hi = p.B;
   while (hi - lo > 1) {
     const int mid = (lo + hi) >> 1;
-    if (p.cu[mid] / p.seg + mid <= z) lo = mid;
+    if ((cs_pos(p, mid) - p.w0) / p.seg + mid <= z) lo = mid;
     else hi = mid;
   }
   s.b = lo;
-  const long long first = p.cu[lo], at = first + (long long)(z - ((int)first / p.seg + lo)) * p.seg;
-  const int end = p.cu[lo + 1];
+  const long long first = cs_pos(p, lo), at = first + (long long)(z - (((int)first - p.w0) / p.seg + lo)) * p.seg;
+  const int end = cs_pos(p, lo + 1);
   s.t0 = at < first || at >= end ? end : (int)at;
   s.t1 = min(end, (int)min((long long)end, s.t0 + (long long)p.seg));
   return s;
 }
 
-// A chunk's place in the record array: unique and increasing over (sequence, chunk), below T / 16 + B + 1.
-__device__ __forceinline__ int cs_slot(int t, int b) { return t / CS_C + b; }
+// A chunk's place in the record array: unique and increasing over (sequence, chunk), below (tokens of the window) / 16 + B + 1.
+__device__ __forceinline__ int cs_slot(const CsParams& p, int t, int b) { return (t - p.w0) / CS_C + b; }
+
+// States in front of and behind this window's part of sequence b, head h; null: zeros, nobody asks.
+__device__ __forceinline__ const float* cs_state_in(const CsParams& p, int b, int h, long long size) {
+  if (p.state) return p.state + ((long long)b * p.H + h) * size;
+  return p.cu[b] < p.w0 ? p.carry_in + h * size : nullptr;
+}
+__device__ __forceinline__ float* cs_state_out(const CsParams& p, int b, int h, long long size) {
+  if (p.state) return p.state + ((long long)b * p.H + h) * size;
+  return p.cu[b + 1] > p.w1 ? p.carry_out + h * size : nullptr;
+}
 
 __device__ __forceinline__ float cs_softplus(float x) { return x > 20.f ? x : log1pf(expf(x)); }
 
@@ -211,11 +228,11 @@ __global__ void __launch_bounds__(128) chunk_coef_kernel(const CsParams p, int h
   int lo = 0, hi = p.B;                 // the last sequence whose first chunk is not past this slot
   while (hi - lo > 1) {
     const int mid = (lo + hi) >> 1;
-    if (cs_slot(p.cu[mid], mid) <= slot) lo = mid;
+    if (cs_slot(p, cs_pos(p, mid), mid) <= slot) lo = mid;
     else hi = mid;
   }
-  const int first = p.cu[lo], end = p.cu[lo + 1];
-  const int t0 = first + (slot - cs_slot(first, lo)) * CS_C;
+  const int first = cs_pos(p, lo), end = cs_pos(p, lo + 1);
+  const int t0 = first + (slot - cs_slot(p, first, lo)) * CS_C;
   if (t0 < first || t0 >= end) return;
   const int n = min(CS_C, end - t0);
   const int rows = h0 / (p.H / p.G);
@@ -390,7 +407,7 @@ __global__ void __launch_bounds__(CS_THREADS) chunk_scan_kernel(const CsParams p
             on ? p.v[((long long)(tb + t) * H + h) * DV + cta_col + c] : __float2bfloat16(0.f);
       }
     }
-    const uint8_t* rec = p.rec + ((long long)cs_slot(tb, b) * H + h) * C::REC;
+    const uint8_t* rec = p.rec + ((long long)cs_slot(p, tb, b) * H + h) * C::REC;
     for (int i = tid; i < C::REC / 16; i += CS_THREADS) cs_copy16(dst + C::OFF_R + i * 16, rec + i * 16, true);
   };
   auto commit = [] { asm volatile("cp.async.commit_group;" ::: "memory"); };
@@ -402,8 +419,8 @@ __global__ void __launch_bounds__(CS_THREADS) chunk_scan_kernel(const CsParams p
 
   // S^T in the accumulator layout: S[nt][e] is row 8 nt + 2 quad + (e & 1) of the state, column col + 8 (e >> 1)
   float S[NT][4];
-  float* pool = p.seg ? p.seg_state + ((long long)span.slot * H + h) * DK * DV
-                      : (p.state ? p.state + ((long long)b * H + h) * DK * DV : nullptr);
+  float* const at_seg = p.seg ? p.seg_state + ((long long)span.slot * H + h) * DK * DV : nullptr;
+  const float* pool = p.seg ? at_seg : cs_state_in(p, b, h, (long long)DK * DV);
   float decay = 1.f;
   const long long row_step = MODE == CS_SSD ? 1 : DV, col_step = MODE == CS_SSD ? DK : 1;
 #pragma unroll
@@ -567,13 +584,14 @@ __global__ void __launch_bounds__(CS_THREADS) chunk_scan_kernel(const CsParams p
     st = st == CS_STAGES - 1 ? 0 : st + 1;
   }
   if (LOCAL && blockIdx.x == 0 && tid == 0) p.seg_decay[(long long)span.slot * H + h] = decay;
-  if (pool && (LOCAL || p.seg == 0)) {
+  float* const left = LOCAL ? at_seg : p.seg ? nullptr : cs_state_out(p, b, h, (long long)DK * DV);
+  if (left) {
 #pragma unroll
     for (int i = 0; i < NT; ++i)
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         const int c = col + 8 * (e >> 1);
-        if (c < DV) pool[(8 * i + 2 * quad + (e & 1)) * row_step + c * col_step] = S[i][e];
+        if (c < DV) left[(8 * i + 2 * quad + (e & 1)) * row_step + c * col_step] = S[i][e];
       }
   }
 }
@@ -582,31 +600,33 @@ __global__ void __launch_bounds__(CS_THREADS) chunk_scan_kernel(const CsParams p
 __global__ void chunk_carry_kernel(const CsParams p, int n4) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x, h = blockIdx.y, b = blockIdx.z;
   if (i >= n4) return;
-  const int first = p.cu[b], n = (p.cu[b + 1] - first + p.seg - 1) / p.seg, slot = first / p.seg + b;
+  const int first = cs_pos(p, b), n = (cs_pos(p, b + 1) - first + p.seg - 1) / p.seg, slot = (first - p.w0) / p.seg + b;
   if (n <= 0) return;
-  float4* pool = p.state ? reinterpret_cast<float4*>(p.state) + ((long long)b * p.H + h) * n4 + i : nullptr;
+  const float4* in = reinterpret_cast<const float4*>(cs_state_in(p, b, h, 4LL * n4));
+  float4* left = reinterpret_cast<float4*>(cs_state_out(p, b, h, 4LL * n4));
   float4* at = reinterpret_cast<float4*>(p.seg_state) + ((long long)slot * p.H + h) * n4 + i;
   const float* decay = p.seg_decay + (long long)slot * p.H + h;
   const long long step = (long long)p.H * n4;
-  float4 s = pool ? *pool : make_float4(0.f, 0.f, 0.f, 0.f), next = at[0];
+  float4 s = in ? in[i] : make_float4(0.f, 0.f, 0.f, 0.f), next = at[0];
   for (int k = 0; k < n; ++k) {
-    const float4 left = next;
+    const float4 own = next;
     if (k + 1 < n) next = at[(k + 1) * step];
     const float d = decay[(long long)k * p.H];
     at[k * step] = s;
-    s = make_float4(fmaf(d, s.x, left.x), fmaf(d, s.y, left.y), fmaf(d, s.z, left.z), fmaf(d, s.w, left.w));
+    s = make_float4(fmaf(d, s.x, own.x), fmaf(d, s.y, own.y), fmaf(d, s.z, own.z), fmaf(d, s.w, own.w));
   }
-  if (pool) *pool = s;
+  if (left) left[i] = s;
 }
 
 template <int MODE, int DK>
-int run_chunk_scan(const CsParams& p, cudaStream_t s) {
+int run_chunk_window(const CsParams& p, cudaStream_t s) {
   int per = 1;                          // heads that share a chunk's products
   if (MODE == CS_SSD)
     while (per < 8 && (p.H / p.G) % (2 * per) == 0) per *= 2;
-  chunk_coef_kernel<MODE, DK><<<dim3(p.T / CS_C + p.B + 1, (p.H / per + 3) / 4), 128, 0, s>>>(p, per);
+  const int tokens = p.w1 - p.w0;
+  chunk_coef_kernel<MODE, DK><<<dim3(tokens / CS_C + p.B + 1, (p.H / per + 3) / 4), 128, 0, s>>>(p, per);
   if (check_cuda(cudaGetLastError(), "chunk_coef launch")) return -1;
-  const int tiles = (p.DV + CS_CT - 1) / CS_CT, spans = p.seg ? p.T / p.seg + p.B + 1 : p.B;
+  const int tiles = (p.DV + CS_CT - 1) / CS_CT, spans = p.seg ? tokens / p.seg + p.B + 1 : p.B;
   if constexpr (MODE == CS_SSD) {
     if (p.seg) {
       chunk_scan_kernel<MODE, DK, true><<<dim3(tiles, p.H, spans), CS_THREADS, 0, s>>>(p);
@@ -620,9 +640,25 @@ int run_chunk_scan(const CsParams& p, cudaStream_t s) {
   return check_cuda(cudaGetLastError(), "chunk_scan launch");
 }
 
+template <int MODE, int DK>
+int run_chunk_scan(CsParams p, int window, float* carry, cudaStream_t s) {
+  const long long size = (long long)p.H * DK * p.DV;
+  for (long long w = 0, i = 0; w < p.T; w += window, ++i) {
+    p.w0 = (int)w;
+    p.w1 = (int)(w + window < p.T ? w + window : p.T);
+    if (carry) p.carry_in = carry + (i & 1) * size, p.carry_out = carry + ((i + 1) & 1) * size;
+    if (run_chunk_window<MODE, DK>(p, s)) return -1;
+  }
+  return 0;
+}
+
 bool cs_aligned(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
-int cs_check(const char* who, CsParams& p, int DK) {
+int cs_check(const char* who, CsParams& p, int DK, int window, const float* carry) {
+  if (window < CS_C || window % CS_C || (window < p.T && !p.state && (!carry || !cs_aligned(carry)))) {
+    set_last_error("%s: a window of %d tokens", who, window);
+    return -1;
+  }
   if (p.H < 1 || p.H > 65535 || p.B > 65535 || p.DV < 1 || p.DV > 256 || !p.rec || !cs_aligned(p.rec) || !cs_aligned(p.q) ||
       !cs_aligned(p.k) || (DK & 15)) {
     set_last_error("%s: sizes (B=%d, H=%d, DK=%d, DV=%d) or unaligned operands", who, p.B, p.H, DK, p.DV);
@@ -638,36 +674,38 @@ int cs_check(const char* who, CsParams& p, int DK) {
 using namespace edl;
 
 // q, k [T, H, DK], v [T, H, DV], beta [T, H] or null: bf16; g fp32 [T, H] or null; state fp32 [nseq, H, DK, DV] or null; o bf16
-// [T, H, DV]; rec: workspace of (T / 16 + nseq + 1) * H * 3344 bytes. DK 32, 64 or 128, DV up to 256.
+// [T, H, DV]. window: tokens taken at a time, a multiple of 16; rec: workspace of (min(window, T) / 16 + nseq + 1) * H * 3344
+// bytes; carry: without a state and with more tokens than a window, two states of one sequence. DK 32, 64 or 128, DV up to 256.
 EDL_HOST_API int edl_delta_rule_chunks(const void* q, const void* k, const void* v, const float* g, const void* beta,
                                        const int* cu, int T, int nseq, int H, int DK, int DV, float scale, float* state, void* o,
-                                       void* rec, void* stream) {
+                                       void* rec, int window, float* carry, void* stream) {
   if (nseq <= 0 || H <= 0 || T <= 0) return 0;
   CsParams p{};
   p.q = (const __nv_bfloat16*)q; p.k = (const __nv_bfloat16*)k; p.v = (const __nv_bfloat16*)v; p.g = g;
   p.beta = (const __nv_bfloat16*)beta; p.cu = cu; p.T = T; p.B = nseq; p.H = p.G = H; p.DV = DV; p.scale = scale;
   p.rec = (uint8_t*)rec; p.state = state; p.o = (__nv_bfloat16*)o;
-  if (cs_check("edl_delta_rule_chunks", p, DK)) return -1;
+  if (cs_check("edl_delta_rule_chunks", p, DK, window, carry)) return -1;
   cudaStream_t s = (cudaStream_t)stream;
   switch (DK) {
-    case 32: return run_chunk_scan<CS_DELTA, 32>(p, s);
-    case 64: return run_chunk_scan<CS_DELTA, 64>(p, s);
-    case 128: return run_chunk_scan<CS_DELTA, 128>(p, s);
+    case 32: return run_chunk_scan<CS_DELTA, 32>(p, window, carry, s);
+    case 64: return run_chunk_scan<CS_DELTA, 64>(p, window, carry, s);
+    case 128: return run_chunk_scan<CS_DELTA, 128>(p, window, carry, s);
   }
   set_last_error("edl_delta_rule_chunks: key head_dim %d not in {32, 64, 128}", DK);
   return -1;
 }
 
 // x [T, H, P], dt [T, H], B, C [T, G, N]: bf16; A, D, dt_bias fp32 [H] (D, dt_bias or null); state fp32 [nseq, H, P, N] or
-// null; y bf16 [T, H, P]; rec: workspace of (T / 16 + nseq + 1) * H * 1680 bytes. N 16, 32, 64 or 128, P up to 256.
-// seg: tokens of a segment (a multiple of 16) or 0; segments: workspace of (T / seg + nseq + 1) * H * (P * N + 1) floats,
-// 16-byte aligned, as `state` has to be then.
+// null; y bf16 [T, H, P]; window, rec (1680 bytes per place), carry: as above. N 16, 32, 64 or 128, P up to 256.
+// seg: tokens of a segment (a multiple of 16) or 0; segments: workspace of (min(window, T) / seg + nseq + 1) * H * (P * N + 1)
+// floats, 16-byte aligned, as `state` has to be then.
 EDL_HOST_API int edl_ssd_scan_chunks(const void* x, const void* dt, const float* A, const void* B, const void* C,
                                      const float* D, const float* dt_bias, int softplus, const int* cu, int T, int nseq, int H,
-                                     int P, int G, int N, float* state, void* y, void* rec, int seg, float* segments,
-                                     void* stream) {
+                                     int P, int G, int N, float* state, void* y, void* rec, int window, float* carry,
+                                     int seg, float* segments, void* stream) {
   if (nseq <= 0 || H <= 0 || T <= 0) return 0;
-  if (seg < 0 || seg % CS_C || (seg && (!segments || !cs_aligned(segments) || !cs_aligned(state) || T / seg + nseq + 1 > 65535))) {
+  const int tokens = window < T ? window : T;            // at a time
+  if (seg < 0 || seg % CS_C || (seg && (!segments || !cs_aligned(segments) || !cs_aligned(state) || tokens / seg + nseq + 1 > 65535))) {
     set_last_error("edl_ssd_scan_chunks: segments of %d tokens", seg);
     return -1;
   }
@@ -681,14 +719,14 @@ EDL_HOST_API int edl_ssd_scan_chunks(const void* x, const void* dt, const float*
   p.scale = 1.f; p.rec = (uint8_t*)rec; p.state = state; p.o = (__nv_bfloat16*)y;
   p.seg = seg;
   p.seg_state = segments;
-  if (seg) p.seg_decay = segments + (long long)(T / seg + nseq + 1) * H * P * N;
-  if (cs_check("edl_ssd_scan_chunks", p, N)) return -1;
+  if (seg) p.seg_decay = segments + (long long)(tokens / seg + nseq + 1) * H * P * N;
+  if (cs_check("edl_ssd_scan_chunks", p, N, window, carry)) return -1;
   cudaStream_t s = (cudaStream_t)stream;
   switch (N) {
-    case 16: return run_chunk_scan<CS_SSD, 16>(p, s);
-    case 32: return run_chunk_scan<CS_SSD, 32>(p, s);
-    case 64: return run_chunk_scan<CS_SSD, 64>(p, s);
-    case 128: return run_chunk_scan<CS_SSD, 128>(p, s);
+    case 16: return run_chunk_scan<CS_SSD, 16>(p, window, carry, s);
+    case 32: return run_chunk_scan<CS_SSD, 32>(p, window, carry, s);
+    case 64: return run_chunk_scan<CS_SSD, 64>(p, window, carry, s);
+    case 128: return run_chunk_scan<CS_SSD, 128>(p, window, carry, s);
   }
   set_last_error("edl_ssd_scan_chunks: state size %d not in {16, 32, 64, 128}", N);
   return -1;

@@ -21,8 +21,8 @@ _lib.register("edl_selective_scan", i32, [vp, vp, vp, vp, vp, vp, vp, vp, i32, v
 _lib.register("edl_ssd_scan", i32, [vp, vp, vp, vp, vp, vp, vp, i32, vp, i32, i32, i32, i32, i32, vp, vp, vp])
 _lib.register("edl_delta_rule", i32, [vp, vp, vp, vp, vp, i32, vp, i32, i32, i32, i32, f32, vp, vp, vp])
 _lib.register("edl_delta_rule_blocks", i32, [vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, f32, vp, vp, vp, vp])
-_lib.register("edl_delta_rule_chunks", i32, [vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, f32, vp, vp, vp, vp])
-_lib.register("edl_ssd_scan_chunks", i32, [vp, vp, vp, vp, vp, vp, vp, i32, vp, i32, i32, i32, i32, i32, i32, vp, vp, vp, i32, vp, vp])
+_lib.register("edl_delta_rule_chunks", i32, [vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, f32, vp, vp, vp, i32, vp, vp])
+_lib.register("edl_ssd_scan_chunks", i32, [vp, vp, vp, vp, vp, vp, vp, i32, vp, i32, i32, i32, i32, i32, i32, vp, vp, vp, i32, vp, i32, vp, vp])
 _lib.register("edl_ragged_conv1d", i32, [vp, vp, vp, vp, vp, i32, i32, i32, i32, vp, vp, vp])
 _lib.register("edl_hgrn2_scan", i32, [vp, i32, _lib.i64, vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, vp, vp, vp])
 _lib.register("edl_hgrn2_decode", i32, [vp, i32, _lib.i64, vp, vp, vp, vp, vp, vp, f32, vp, i32, i32, i32, i32, vp])
@@ -47,6 +47,9 @@ def _use_kernel(*ts) -> bool:
         x is not None and x.requires_grad for x in ts))
 
 
+SCAN_WORKSPACE = 256 << 20        # bytes of records at a time
+
+
 def _scan_records(total: int, nseq: int, heads: int, chunk: int, size: int, *rows: torch.Tensor) -> torch.Tensor | None:
     """Workspace (``size`` bytes per chunk and head) of the scans that take ``chunk`` tokens at a time (``csrc/chunk_scan.cu``
     sixteen, ``csrc/block_scan.cu`` eight), or None where the one-token kernels run: rows that do not start on 16 bytes, and
@@ -54,14 +57,27 @@ def _scan_records(total: int, nseq: int, heads: int, chunk: int, size: int, *row
     saves: 16 heads of 128 x 128, chunks against tokens, 64 sequences of 1, 2, 4, 8 tokens 48, 50, 52, 52 us against 51, 74,
     118, 212 (state space of 64 x 128: 38, 38, 38, 40 against 81, 83, 87, 98); one sequence of 4 or 16 tokens 34, 34 us against
     24, 54. A block on the FMA pipe costs the same for one token as for eight: with a decay per channel, blocks against
-    tokens, the same steps 88, 89, 81, 85 us against 58, 88, 148, 274."""
+    tokens, the same steps 88, 89, 81, 85 us against 58, 88, 148, 274. Every sequence has a chunk of its own; so many that those
+    take four times SCAN_WORKSPACE fill the GPU token by token."""
     if chunk == 16:
         few = total < 8 * nseq and nseq * heads < 1024
     else:
         few = total < 4 * nseq
-    if few or any(t.data_ptr() % 16 for t in rows):
+    if few or (nseq + 1) * heads * size > 4 * SCAN_WORKSPACE or any(t.data_ptr() % 16 for t in rows):
         return None
-    return torch.empty((total // chunk + nseq + 1) * heads * size, dtype=torch.uint8, device=rows[0].device)
+    tokens = min(total, _scan_window(heads, size)) if chunk == 16 else total
+    return torch.empty((tokens // chunk + nseq + 1) * heads * size, dtype=torch.uint8, device=rows[0].device)
+
+
+def _scan_window(heads: int, size: int) -> int:
+    """Tokens that the scans of sixteen at a time take per launch: what SCAN_WORKSPACE holds records of. Longer inputs go in
+    windows, with the state of the sequence that a window's end cuts in front of the next one."""
+    return max(1024, SCAN_WORKSPACE // (heads * size) * 16 // 1024 * 1024)
+
+
+def _scan_carry(total: int, window: int, state, shape: tuple[int, ...], device) -> torch.Tensor | None:
+    """Where the sequences that windows cut keep their states if the caller does not."""
+    return torch.empty(2, *shape, dtype=torch.float32, device=device) if state is None and window < total else None
 
 
 def _scan_segment(total: int, nseq: int, units: int, size: int) -> int:
@@ -276,7 +292,10 @@ def ssd_scan_chunked(x, dt, A, B, C, D=None, dt_bias=None, softplus=True, cu_seq
 
 
 def ssd_scan(x, dt, A, B, C, D=None, dt_bias=None, softplus=True, cu_seqlens=None, state=None):
-    """x ``[total, H, P]``; dt ``[total, H]``; A ``[H]``; B, C ``[total, G, N]``; state ``[nseq, H, P, N]`` fp32."""
+    """x ``[total, H, P]``; dt ``[total, H]``; A ``[H]``; B, C ``[total, G, N]``; state ``[nseq, H, P, N]`` fp32.
+
+    The kernels keep a workspace of 105 bytes per token and head, at most SCAN_WORKSPACE, besides 1680 per sequence and head.
+    A value that is not finite reaches outputs from its token on only."""
     if _use_kernel(x, dt, A, B, C, D) and B.shape[2] in (16, 32, 64, 128) and x.dtype == torch.bfloat16 \
             and x.shape[2] <= 256:
         total, H, P = x.shape
@@ -291,10 +310,13 @@ def ssd_scan(x, dt, A, B, C, D=None, dt_bias=None, softplus=True, cu_seqlens=Non
         args = (x.data_ptr(), dt.data_ptr(), A.data_ptr(), B.data_ptr(), C.data_ptr(), _lib.ptr(D), _lib.ptr(dt_bias),
                 int(softplus), cu.data_ptr())
         if rec is not None:
-            seg = _scan_segment(total, nseq, H * ((P + 63) // 64), N) if state is None or state.data_ptr() % 16 == 0 else 0
-            parts = torch.empty((total // seg + nseq + 1) * H * (P * N + 1), dtype=torch.float32, device=x.device) if seg else None
-            _lib.call("edl_ssd_scan_chunks", *args, total, nseq, H, P, G, N, _lib.ptr(state), y.data_ptr(), rec.data_ptr(), seg,
-                      _lib.ptr(parts), _lib.stream_ptr())
+            window = _scan_window(H, 1680)
+            tokens = min(total, window)
+            seg = _scan_segment(tokens, nseq, H * ((P + 63) // 64), N) if state is None or state.data_ptr() % 16 == 0 else 0
+            parts = torch.empty((tokens // seg + nseq + 1) * H * (P * N + 1), dtype=torch.float32, device=x.device) if seg else None
+            carry = _scan_carry(total, window, state, (H, P, N), x.device)
+            _lib.call("edl_ssd_scan_chunks", *args, total, nseq, H, P, G, N, _lib.ptr(state), y.data_ptr(), rec.data_ptr(), window,
+                      _lib.ptr(carry), seg, _lib.ptr(parts), _lib.stream_ptr())
         else:
             _lib.call("edl_ssd_scan", *args, nseq, H, P, G, N, _lib.ptr(state), y.data_ptr(), _lib.stream_ptr())
         return y
@@ -377,8 +399,10 @@ def gated_delta_rule(q, k, v, g=None, beta=None, scale=None, cu_seqlens=None, st
     """q, k ``[total, H, DK]``; v ``[total, H, DV]``; g ``[total, H]`` log-decay (or ``[total, H, DK]`` for KDA);
     beta ``[total, H]``; state ``[nseq, H, DK, DV]`` fp32. Returns ``[total, H, DV]``.
 
-    Inference on the GPU runs the recurrent kernel; anything that needs gradients (or long CPU inputs) with a
-    per-head gate goes through :func:`delta_rule_chunked`."""
+    Inference on the GPU runs the recurrent kernels, with a workspace of 209 bytes per token and head (at most SCAN_WORKSPACE,
+    besides 3344 per sequence and head; with a decay per channel 36 per token, without a bound, and 288); a value that is not
+    finite reaches outputs from its token on only. Anything that needs gradients (or long CPU inputs) with a per-head gate goes
+    through :func:`delta_rule_chunked`."""
     DK, DV = q.shape[-1], v.shape[-1]
     if _use_kernel(q, k, v, g, beta) and DK in (32, 64, 128) and DV <= 256 and q.dtype == torch.bfloat16:
         total, H, _ = q.shape
@@ -391,9 +415,14 @@ def gated_delta_rule(q, k, v, g=None, beta=None, scale=None, cu_seqlens=None, st
         scale = float(scale if scale is not None else DK ** -0.5)
         args = (q.data_ptr(), k.data_ptr(), v.data_ptr(), _lib.ptr(g), _lib.ptr(beta))
         rec = _scan_records(total, nseq, H, 8, 288, q, k, g) if per_channel else _scan_records(total, nseq, H, 16, 3344, q, k)
-        if rec is not None:
-            _lib.call("edl_delta_rule_blocks" if per_channel else "edl_delta_rule_chunks", *args, cu.data_ptr(), total, nseq, H, DK,
-                      DV, scale, _lib.ptr(state), o.data_ptr(), rec.data_ptr(), _lib.stream_ptr())
+        if rec is not None and per_channel:
+            _lib.call("edl_delta_rule_blocks", *args, cu.data_ptr(), total, nseq, H, DK, DV, scale, _lib.ptr(state), o.data_ptr(),
+                      rec.data_ptr(), _lib.stream_ptr())
+        elif rec is not None:
+            window = _scan_window(H, 3344)
+            carry = _scan_carry(total, window, state, (H, DK, DV), q.device)
+            _lib.call("edl_delta_rule_chunks", *args, cu.data_ptr(), total, nseq, H, DK, DV, scale, _lib.ptr(state), o.data_ptr(),
+                      rec.data_ptr(), window, _lib.ptr(carry), _lib.stream_ptr())
         else:
             _lib.call("edl_delta_rule", *args, per_channel, cu.data_ptr(), nseq, H, DK, DV, scale, _lib.ptr(state), o.data_ptr(),
                       _lib.stream_ptr())

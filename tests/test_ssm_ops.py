@@ -109,6 +109,32 @@ def test_scans_keep_what_is_not_finite_from_earlier_tokens(what, at):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("with_state", [True, False])
+@pytest.mark.parametrize("cu", [[0, 5000], [0, 700, 1024, 1025, 1025, 3500, 5000], [0, 1024, 2048, 5000], [3, 40, 4990]])
+def test_scans_in_windows_give_what_one_pass_gives(cu, with_state, monkeypatch):
+    """Inputs longer than the workspace holds records of: sequences cut by windows of 1024 tokens once, several times or at a
+    window's end, with the caller's states and with their own; segments inside windows (the state space with few heads)."""
+    torch.manual_seed(len(cu))
+    dev, T, H, D, n = "cuda", 5000, 2, 64, len(cu) - 1
+    cu = torch.tensor(cu, dtype=torch.int32, device=dev)
+    rnd = lambda *s: torch.randn(*s, device=dev)
+    q, k = (torch.nn.functional.normalize(rnd(T, H, D), dim=-1).to(torch.bfloat16) for _ in range(2))
+    v, g, beta = rnd(T, H, D).to(torch.bfloat16), -0.1 * torch.rand(T, H, device=dev), torch.rand(T, H, device=dev).to(torch.bfloat16)
+    B, C, dt = rnd(T, 1, D).to(torch.bfloat16), rnd(T, 1, D).to(torch.bfloat16), (rnd(T, H) - 3).to(torch.bfloat16)
+    A, Dv = -torch.rand(H, device=dev) - 0.5, rnd(H)
+    got = []
+    for limit in (ssm.SCAN_WORKSPACE, 1 << 14):
+        monkeypatch.setattr(ssm, "SCAN_WORKSPACE", limit)
+        states = [torch.ones(n, H, D, D, device=dev) if with_state else None for _ in range(2)]
+        o = ssm.gated_delta_rule(q, k, v, g, beta, None, cu, states[0])
+        y = ssm.ssd_scan(v, dt, A, B, C, Dv, None, True, cu, states[1])
+        got.append([t[int(cu[0]):int(cu[-1])].float() for t in (o, y)] + [s for s in states if s is not None])
+    assert ssm._scan_window(H, 1680) == 1024
+    for i, (a, b) in enumerate(zip(*got)):      # outputs are rounded to bf16 once, states are fp32 sums in another order
+        assert (a - b).abs().max() <= (2.0 ** -7 if i < 2 else 1e-5) * b.abs().max(), i
+
+
+@pytest.mark.gpu
 def test_ragged_conv1d_cuda():
     torch.manual_seed(4)
     dev, T, Cn, W = "cuda", 50, 96, 4
