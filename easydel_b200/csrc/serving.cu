@@ -154,7 +154,8 @@ __device__ __forceinline__ void row_values(const SampleArgs& a, const char* rowp
 
 // One row of logits per cluster of CTAs, a slice of the row per CTA. Greedy rows (temperature <= 0 or top_k == 1) take
 // the arg-max of the penalised logits. Other rows take the `top_k` (<= 64) best candidates, apply temperature, top-p and
-// min-p to them and draw one with a counter-based RNG keyed by (seed[row], step[row]).
+// min-p to them and draw one with a counter-based RNG keyed by (seed[row], step[row]). A row without a value above minus
+// infinity gives token 0 with log-probability minus infinity.
 //
 // What bounds it is the latency of a few passes over a slice, so the row is read once: every thread keeps the maximum (and
 // the online sum of exponentials) of its own values. The k-th largest of those maxima, found bit by bit with block-wide
@@ -358,10 +359,9 @@ __global__ void __launch_bounds__(SAMP_THREADS, 2) sample_kernel(const SampleArg
   }
   if (greedy) {
     if (tid == 0) {
-      int i = cand_i[0];
-      if (N > 1 && !pen && cand_v[0] == -INFINITY) i = 0x7fffffff;      // nothing above minus infinity in the row
-      a.out[row] = i;
-      if (a.out_logprob) a.out_logprob[row] = cand_v[0] - lse;
+      const bool none = cand_v[0] == -INFINITY;      // nothing above minus infinity in the row, as for sampled rows below
+      a.out[row] = none ? 0 : cand_i[0];
+      if (a.out_logprob) a.out_logprob[row] = none ? -INFINITY : cand_v[0] - lse;
     }
     return;
   }

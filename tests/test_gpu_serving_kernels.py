@@ -361,3 +361,27 @@ def test_sampler_draws_what_the_oracle_draws(R, V, form):
                 continue
             assert int(tok[r]) == want, (r, k)
             assert abs(float(lp[r]) - want_lp) < 1e-4 * max(1.0, abs(want_lp))
+
+
+@pytest.mark.parametrize("V", [1000, 1003, 40000])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("penalties", [False, True])
+@pytest.mark.parametrize("temperature", [0.0, 0.7])
+def test_sampler_on_rows_without_a_usable_value(V, dtype, penalties, temperature):
+    """Rows of minus infinities, of NaNs and of both give token 0 with log-probability minus infinity in every form of the
+    kernel (16-byte loads or not, a row cut over a cluster, penalties); one finite value among them is taken."""
+    from easydel_b200.ops import serving as S
+
+    inf = float("inf")
+    logits = torch.full((5, V), -inf, device="cuda")
+    logits[1] = float("nan")
+    logits[2, ::2] = float("nan")
+    logits[3, V - 2] = -3.0
+    logits[4] = float("nan")
+    logits[4, 17] = 2.0
+    kw = dict(temperature=torch.full((5,), temperature, device="cuda"))
+    if penalties:
+        kw.update(counts=torch.ones(5, V, dtype=torch.int32, device="cuda"), presence=torch.full((5,), 0.5, device="cuda"))
+    tokens, logprobs = S.sample(logits.to(dtype), want_logprob=True, **kw)
+    assert tokens.tolist() == [0, 0, 0, V - 2, 17]
+    assert (logprobs[:3] == -inf).all() and abs(float(logprobs[3])) < 1e-5
