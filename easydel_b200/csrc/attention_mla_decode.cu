@@ -14,7 +14,8 @@
 //     the output needs no merge across warps;
 //   * with key splits the partial outputs and log-sum-exps are merged by edl_attn_combine.
 // L and R are multiples of 8 with L + R <= 64 NB and L <= 512.
-// Many heads and long sequences go to the tcgen05 form further down, one CTA per 128 heads and half of the value columns.
+// Many heads and long sequences go to the tcgen05 form further down, one CTA per 128 heads and half of the value columns; where
+// the CTAs of both forms fit the GPU at once, the length of each sequence decides on the device.
 //
 // Role of the reference's multi-latent ragged page attention for decode steps
 // (easydel/operations/kernels/multi_latent_ragged_page_attention.py:282-700).
@@ -88,18 +89,18 @@ __device__ __forceinline__ uint32_t ml_tile_off(int row, int chunk) {
   return box * (ML_TK * 128) + row * 128 + ((c ^ (row & 7)) << 4);
 }
 
+// The first four warps meet; the tcgen05 form's CTAs have six.
+__device__ __forceinline__ void ml_sync() { asm volatile("bar.sync 1, %0;" ::"n"(ML_THREADS) : "memory"); }
+
 template <int NB>
-__global__ void __launch_bounds__(ML_THREADS, NB > 4 ? 1 : 2)
-mla_decode_kernel(const __grid_constant__ CUtensorMap tmap, const MlaParams p) {
+__device__ __forceinline__ void mla_decode_simple(const CUtensorMap& tmap, const MlaParams& p, uint8_t* smem, int id) {
   using C = MlCfg<NB>;
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const uint32_t sbase = smem_u32(smem);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int groups = (p.H + 15) / 16;
-  const int split = blockIdx.x % p.splits;
-  const int hg = (blockIdx.x / p.splits) % groups;
-  const int b = blockIdx.x / (p.splits * groups);
+  const int split = id % p.splits;
+  const int hg = (id / p.splits) % groups;
+  const int b = id / (p.splits * groups);
   const int heads = min(16, p.H - hg * 16);
   const int kv_len = p.kv_lens[b];
   const int* pt = p.page_table + (long long)b * p.pt_stride;
@@ -112,10 +113,10 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tmap, const MlaParams p) {
 
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::OFF_BAR);
   const uint32_t bar0 = smem_u32(bars);
-  __shared__ int s_abort;
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + C::OFF_BAR + 8 * ML_STAGES);
   if (threadIdx.x == 0) {
     for (int i = 0; i < ML_STAGES; ++i) mbar_init(bar0 + 8 * i, 1);
-    s_abort = 0;
+    *abort_flag = 0;
     fence_mbar_init();
     prefetch_tmap(&tmap);
   }
@@ -130,8 +131,7 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tmap, const MlaParams p) {
       *reinterpret_cast<uint4*>(smem + C::OFF_Q + r * C::QPITCH + c * 2) = v;
     }
   }
-  __syncthreads();
-  volatile int* abort_flag = &s_abort;
+  ml_sync();
 
   auto issue = [&](int i) {  // thread 0 only
     const int tile = t0 + i;
@@ -211,7 +211,7 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tmap, const MlaParams p) {
       s_max[(par * ML_WARPS + warp) * 16 + r0] = mx[0];
       s_max[(par * ML_WARPS + warp) * 16 + r0 + 8] = mx[1];
     }
-    __syncthreads();
+    ml_sync();
     float alpha[2];
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
@@ -231,7 +231,7 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tmap, const MlaParams p) {
       *reinterpret_cast<uint32_t*>(pb + r0 * ML_PPITCH) = pack_bf16x2(e0, e1);
       *reinterpret_cast<uint32_t*>(pb + (r0 + 8) * ML_PPITCH) = pack_bf16x2(e2, e3);
     }
-    __syncthreads();
+    ml_sync();
     // ---- O[:, this warp's columns] = O * alpha + P V
 #pragma unroll
     for (int j = 0; j < C::NJ; ++j) {
@@ -269,7 +269,7 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tmap, const MlaParams p) {
     s_sum[warp * 16 + r0] = l_run[0];
     s_sum[warp * 16 + r0 + 8] = l_run[1];
   }
-  __syncthreads();
+  ml_sync();
   const long long orow = (long long)split * p.B + b;
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
@@ -290,11 +290,18 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tmap, const MlaParams p) {
       p.lse[((long long)split * p.H + hg * 16 + r) * p.B + b] =
           l > 0.f ? (m_run[h] + log2f(l)) * 0.6931471805599453f : -INFINITY;
   }
-  if (s_abort) {   // a wait ran out: give copies still in flight time to land before shared memory is released
+  if (*abort_flag) {   // a wait ran out: give copies still in flight time to land before shared memory is released
     long long t0c = clock64();
     while (clock64() - t0c < 400000) {
     }
   }
+}
+
+template <int NB>
+__global__ void __launch_bounds__(ML_THREADS, NB > 4 ? 1 : 2)
+mla_decode_kernel(const __grid_constant__ CUtensorMap tmap, const MlaParams p) {
+  extern __shared__ uint8_t smem_raw[];
+  mla_decode_simple<NB>(tmap, p, reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023)), blockIdx.x);
 }
 
 template <int NB>
@@ -369,16 +376,12 @@ __device__ __forceinline__ float mt_ld_peer(uint32_t addr) {
   return v;
 }
 
-__global__ void __launch_bounds__(MT_THREADS, 1)
-mla_decode_tc_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ CUtensorMap tql,
-                     const __grid_constant__ CUtensorMap tqr, const MlaParams p, const int parts, const int halves,
-                     const int swap_l, const int swap_r) {
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+__device__ __forceinline__ void mla_decode_tc(const CUtensorMap& tmap, const CUtensorMap& tql, const CUtensorMap& tqr,
+                                              const MlaParams& p, const int parts, const int halves, const int swap_l,
+                                              const int swap_r, uint8_t* smem, int id) {
   const uint32_t sbase = smem_u32(smem);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int groups = (p.H + 127) / 128;
-  int id = blockIdx.x;
   const int part = id % parts;
   id /= parts;
   const int half = id % halves;
@@ -758,6 +761,48 @@ mla_decode_tc_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_cons
   if (warp == 1) tmem_dealloc(tmem, 512);
 }
 
+__global__ void __launch_bounds__(MT_THREADS, 1)
+mla_decode_tc_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ CUtensorMap tql,
+                     const __grid_constant__ CUtensorMap tqr, const MlaParams p, const int parts, const int halves,
+                     const int swap_l, const int swap_r) {
+  extern __shared__ uint8_t smem_raw[];
+  mla_decode_tc(tmap, tql, tqr, p, parts, halves, swap_l, swap_r,
+                reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023)), blockIdx.x);
+}
+
+// What either form takes for one round of its CTAs, in us: see mla_takes_tc.
+__host__ __device__ inline float mla_time_simple(long long seen, int splits) {
+  const long long tiles = (seen + ML_TK - 1) / ML_TK;
+  return 5.f + 1.4f * ((tiles + splits - 1) / splits);
+}
+__host__ __device__ inline float mla_time_tc(long long seen, int splits, int parts) {
+  const long long tiles = (seen + MT_TK - 1) / MT_TK, mine = (tiles + splits - 1) / splits;
+  int act = parts;
+  while (act > 1 && mine < act * MT_MIN_TILES) act >>= 1;
+  return (act > 1 ? 12.5f : 10.f) + 2.f * ((mine + act - 1) / act);
+}
+
+// Either form, by the length of the sequence, where the CTAs of both fit the GPU at once: a page table has room for the longest
+// sequence there can be, so the host does not know, and a captured step keeps its launches while the sequences grow. A sequence
+// has `slots` CTAs, as many as the form that needs more of them takes; the others leave.
+template <int NB>
+__global__ void __launch_bounds__(MT_THREADS, 1)
+mla_decode_either_kernel(const __grid_constant__ CUtensorMap tsimple, const __grid_constant__ CUtensorMap tmap,
+                         const __grid_constant__ CUtensorMap tql, const __grid_constant__ CUtensorMap tqr, const MlaParams p,
+                         const int parts, const int halves, const int swap_l, const int swap_r, const int slots) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  const int b = blockIdx.x / slots, i = blockIdx.x - b * slots;
+  const int kv_len = p.kv_lens[b], seen = p.window > 0 ? min(kv_len, p.window) : kv_len;
+  if (mla_time_simple(seen, p.splits) <= mla_time_tc(seen, p.splits, parts)) {
+    const int mine = (p.H + 15) / 16 * p.splits;
+    if (i < mine && threadIdx.x < ML_THREADS) mla_decode_simple<NB>(tsimple, p, smem, b * mine + i);
+  } else {
+    const int mine = (p.H + 127) / 128 * p.splits * halves * parts;
+    if (i < mine) mla_decode_tc(tmap, tql, tqr, p, parts, halves, swap_l, swap_r, smem, b * mine + i);
+  }
+}
+
 // CTAs of a cluster that share a (sequence, 128 heads, half, split): as many as the SMs take at once.
 int mla_parts(const MlaParams& p) {
   const long long ctas = (long long)p.B * ((p.H + 127) / 128) * (p.L > 256 ? 2 : 1) * p.splits;
@@ -768,27 +813,36 @@ int mla_parts(const MlaParams& p) {
 
 // Which form is the faster one, from sizes alone (the table's width bounds the keys): a fixed cost and a time per tile of 32
 // (64) rows, times the rounds the CTAs take. Fitted to both on one B200: the mma.sync form starts in 5 us and takes 1.4 us
-// a tile, this one 10 and 1.8. Where the two are close so are the measurements (16 sequences of 200 to 700 rows, 24 heads,
-// 4 splits: 17.2 against 17.8 us; 64 of 90 to 300, 20 heads: 19.3 against 18.1).
+// a tile, this one 10 (12.5 over a cluster) and 2. Where the two are close so are the measurements (16 sequences of 200 to 700
+// rows, 24 heads, 4 splits: 17.2 against 17.8 us; 64 of 90 to 300, 20 heads: 19.3 against 18.1).
+bool mla_tc_supports(const MlaParams& p) {
+  return (p.L + 63) / 64 + (p.R + 63) / 64 <= MT_MAX_BOXES && !(p.ldo & 7) && !(reinterpret_cast<uintptr_t>(p.o) & 15);
+}
 bool mla_takes_tc(const MlaParams& p) {
-  if ((p.L + 63) / 64 + (p.R + 63) / 64 > MT_MAX_BOXES || (p.ldo & 7) || (reinterpret_cast<uintptr_t>(p.o) & 15)) return false;
   const long long sms = sm_count(), keys = (long long)p.pt_stride * ML_PAGE;
   const long long seen = p.window > 0 && p.window < keys ? p.window : keys;
-  auto up = [](long long a, long long b) { return (a + b - 1) / b; };
+  auto rounds = [&](long long ctas) { return (double)((ctas + sms - 1) / sms); };
   const int parts = mla_parts(p);
-  const long long tiles = up(up(seen, MT_TK), p.splits);
-  int act = parts;
-  while (act > 1 && tiles < act * MT_MIN_TILES) act >>= 1;
-  const double simple = 5.0 + 1.4 * up(up(seen, ML_TK), p.splits) * up((long long)p.B * ((p.H + 15) / 16) * p.splits, sms);
-  const double here =
-      10.0 + 1.8 * up(tiles, act) * up((long long)p.B * ((p.H + 127) / 128) * (p.L > 256 ? 2 : 1) * p.splits * parts, sms);
+  const double simple = 5.0 + (mla_time_simple(seen, p.splits) - 5.0) * rounds((long long)p.B * ((p.H + 15) / 16) * p.splits);
+  const double here = 10.0 + (mla_time_tc(seen, p.splits, parts) - 10.0) *
+                                 rounds((long long)p.B * ((p.H + 127) / 128) * (p.L > 256 ? 2 : 1) * p.splits * parts);
   return here < simple;
 }
+// CTAs of a sequence in the launch that can take either form, 0 where they do not all fit the GPU at once.
+int mla_either_slots(const MlaParams& p) {
+  const int parts = mla_parts(p), halves = p.L > 256 ? 2 : 1;
+  const long long simple = (long long)(p.H + 15) / 16 * p.splits, tc = (long long)(p.H + 127) / 128 * p.splits * halves * parts;
+  const long long slots = ((simple > tc ? simple : tc) + parts - 1) / parts * parts;
+  return slots * p.B <= sm_count() ? (int)slots : 0;
+}
 
+// NB: of the mma.sync form where a launch can take either, else 0.
+template <int NB>
 int launch_mla_tc(const void* pages, long long num_pages, const MlaParams& p, cudaStream_t stream) {
-  CUtensorMap tm, tql, tqr;
+  CUtensorMap ts, tm, tql, tqr;
   const int w = p.L + p.R;
   if (make_tmap_2d_16b(&tm, pages, (uint64_t)num_pages * ML_PAGE, w, w, MT_TK, 64)) return -1;
+  if (NB > 0 && make_tmap_2d_16b(&ts, pages, (uint64_t)num_pages * ML_PAGE, w, w, ML_TK, 64)) return -1;
   // queries as [sequence][head][column] or, where heads lie further apart than sequences, [head][sequence][column]
   const bool swap_l = p.B > 1 && p.q_seq < p.q_head, swap_r = p.B > 1 && p.qr_seq < p.qr_head;
   auto map_q = [&](CUtensorMap* m, const void* base, int cols, long long seq, long long head, bool swap) {
@@ -799,20 +853,23 @@ int launch_mla_tc(const void* pages, long long num_pages, const MlaParams& p, cu
   if (map_q(&tql, p.q, p.L, p.q_seq, p.q_head, swap_l)) return -1;
   tqr = tql;
   if (p.R > 0 && map_q(&tqr, p.qr, p.R, p.qr_seq, p.qr_head, swap_r)) return -1;
+  const void* kern = reinterpret_cast<const void*>(mla_decode_tc_kernel);
+  if constexpr (NB > 0) kern = reinterpret_cast<const void*>(mla_decode_either_kernel<NB>);
   static bool attr_set[64] = {false};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64) dev = 0;
   if (!attr_set[dev]) {
-    if (check_cuda(cudaFuncSetAttribute(mla_decode_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MT_SMEM),
+    if (check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, MT_SMEM),
                    "cudaFuncSetAttribute(mla_decode_tc)"))
       return -1;
     attr_set[dev] = true;
   }
   const int halves = p.L > 256 ? 2 : 1, parts = mla_parts(p);
-  const long long ctas = (long long)p.B * ((p.H + 127) / 128) * halves * p.splits;
+  const long long ctas = (long long)p.B * ((p.H + 127) / 128) * halves * p.splits * parts;
+  const int slots = NB > 0 ? mla_either_slots(p) : 0;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(ctas * parts), 1, 1);
+  cfg.gridDim = dim3((unsigned)(NB > 0 ? (long long)slots * p.B : ctas), 1, 1);
   cfg.blockDim = dim3(MT_THREADS, 1, 1);
   cfg.dynamicSmemBytes = MT_SMEM;
   cfg.stream = stream;
@@ -823,7 +880,20 @@ int launch_mla_tc(const void* pages, long long num_pages, const MlaParams& p, cu
   at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  return check_cuda(cudaLaunchKernelEx(&cfg, mla_decode_tc_kernel, tm, tql, tqr, p, parts, halves, (int)swap_l, (int)swap_r), "mla_decode_tc launch");
+  cudaError_t e;
+  if constexpr (NB > 0)
+    e = cudaLaunchKernelEx(&cfg, mla_decode_either_kernel<NB>, ts, tm, tql, tqr, p, parts, halves, (int)swap_l, (int)swap_r, slots);
+  else
+    e = cudaLaunchKernelEx(&cfg, mla_decode_tc_kernel, tm, tql, tqr, p, parts, halves, (int)swap_l, (int)swap_r);
+  return check_cuda(e, "mla_decode_tc launch");
+}
+
+template <int NB>
+int launch_mla_sized(const void* pages, long long num_pages, const MlaParams& p, cudaStream_t s) {
+  static_assert(MlCfg<NB>::SMEM <= MT_SMEM, "");
+  if (mla_tc_supports(p) && mla_takes_tc(p))
+    return mla_either_slots(p) ? launch_mla_tc<NB>(pages, num_pages, p, s) : launch_mla_tc<0>(pages, num_pages, p, s);
+  return launch_mla<NB>(pages, num_pages, p, s);
 }
 
 }  // namespace
@@ -858,16 +928,15 @@ EDL_HOST_API int edl_attn_mla_decode(const void* q, long long q_seq, long long q
               qr_head, reinterpret_cast<__nv_bfloat16*>(o), ldo, lse, kv_lens, page_table, sinks, pt_stride, B, H, splits,
               L, R, window, scale * ML_LOG2E, status};
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  if (mla_takes_tc(p)) return launch_mla_tc(pages, num_pages, p, s);
   switch ((L + R + 63) / 64) {
-    case 1: return launch_mla<1>(pages, num_pages, p, s);
-    case 2: return launch_mla<2>(pages, num_pages, p, s);
-    case 3: return launch_mla<3>(pages, num_pages, p, s);
-    case 4: return launch_mla<4>(pages, num_pages, p, s);
-    case 5: return launch_mla<5>(pages, num_pages, p, s);
-    case 6: return launch_mla<6>(pages, num_pages, p, s);
-    case 7: return launch_mla<7>(pages, num_pages, p, s);
-    case 8: return launch_mla<8>(pages, num_pages, p, s);
-    default: return launch_mla<9>(pages, num_pages, p, s);
+    case 1: return launch_mla_sized<1>(pages, num_pages, p, s);
+    case 2: return launch_mla_sized<2>(pages, num_pages, p, s);
+    case 3: return launch_mla_sized<3>(pages, num_pages, p, s);
+    case 4: return launch_mla_sized<4>(pages, num_pages, p, s);
+    case 5: return launch_mla_sized<5>(pages, num_pages, p, s);
+    case 6: return launch_mla_sized<6>(pages, num_pages, p, s);
+    case 7: return launch_mla_sized<7>(pages, num_pages, p, s);
+    case 8: return launch_mla_sized<8>(pages, num_pages, p, s);
+    default: return launch_mla_sized<9>(pages, num_pages, p, s);
   }
 }

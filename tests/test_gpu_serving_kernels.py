@@ -276,6 +276,29 @@ def test_latent_decode_many_heads(H, L, R, lens, window, splits):
         assert float((o[b].double() - want).abs().max()) <= tol, (b, n)
 
 
+@pytest.mark.parametrize("H,splits", [(128, 1), (40, 4)])
+def test_latent_decode_of_short_and_long_sequences_under_a_wide_table(H, splits):
+    """A table far wider than the sequences: every sequence takes the form for its own length within one launch. Queries that
+    are one row for all heads, or for all sequences, are views with a pitch of zero."""
+    from easydel_b200.ops import serving as S
+
+    torch.manual_seed(H)
+    lens = [1, 50, 2500, 0, 190, 900]
+    B, need = len(lens), 20
+    pages = (torch.randn(B * need + 1, 128, 1, 576, device="cuda") * 0.5).to(torch.bfloat16)
+    table = torch.zeros(B, 256, dtype=torch.int32, device="cuda")
+    table[:, :need] = (torch.randperm(B * need, device="cuda") + 1).view(B, need)
+    q = (torch.randn(B, H, 576, device="cuda") * 0.5).to(torch.bfloat16)
+    kv = torch.tensor(lens, dtype=torch.int32, device="cuda")
+    for qq in (q, q[:, :1].expand(B, H, 576), q[:1].expand(B, H, 576)):
+        o = S.latent_decode(qq[..., :512], qq[..., 512:], pages, kv, table, scale=0.1, num_splits=splits)
+        for b, n in enumerate(lens):
+            rows = pages[table[b, :need].long()].reshape(-1, 576)[:n].double()
+            want = torch.softmax(qq[b].double() @ rows.T * 0.1, -1) @ rows[:, :512]
+            # as above: probabilities, outputs and partial outputs rounded to bf16
+            assert float((o[b].double() - want).abs().max()) <= 3 * 2.0 ** -8 * float(rows.abs().max() if n else 0), (b, n)
+
+
 @pytest.mark.parametrize("B,H,n", [(32, 128, 600), (4, 128, 2000), (100, 64, 300)])
 def test_latent_decode_of_peaked_scores_keeps_the_output_s_precision(B, H, n):
     """Scores of a standard deviation of 2.25, so that a few keys carry most of a sum and maxima grow along a sequence: what is
