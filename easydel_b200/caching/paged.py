@@ -18,6 +18,8 @@ from dataclasses import dataclass, field
 import torch
 
 from ..ops import serving as S
+from ..ops.kernels import sm_count
+from ..ops.latent import decode_splits as latent_splits
 
 PAGE_SIZE = S.PAGE_SIZE
 
@@ -412,8 +414,8 @@ class PagedLatentView:
         B = meta.num_seqs
         if meta.max_q == 1 and T == B and mla.rope_dim == 64 and L == 512 and S.mla_decode_kernel_supports(q, self.pages):
             # a pure decode step of the 512 + 64 layout: the streaming kernel walks the page table itself
-            o_lat = S.mla_decode_attention(q.contiguous(), self.pages, meta.kv_lens, meta.page_table, scale=mla.scale,
-                                           num_splits=meta.num_splits)
+            n = latent_splits(B, H, None, meta.page_table.shape[1] * S.PAGE_SIZE, sm_count(q.device))
+            o_lat = S.mla_decode_attention(q.contiguous(), self.pages, meta.kv_lens, meta.page_table, scale=mla.scale, num_splits=n)
             return torch.einsum("bhl,hvl->bhv", o_lat, w_uv.to(o_lat.dtype))[None]
         table = meta.page_table[:B].long().clamp_min(0)
         kv = self.pages[table].reshape(B, -1, self.pages.shape[-1])                                       # [B,Tk,L+R]

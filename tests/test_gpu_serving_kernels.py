@@ -299,6 +299,29 @@ def test_latent_decode_of_short_and_long_sequences_under_a_wide_table(H, splits)
             assert float((o[b].double() - want).abs().max()) <= 3 * 2.0 ** -8 * float(rows.abs().max() if n else 0), (b, n)
 
 
+def test_latent_view_plans_its_own_splits():
+    """The step's key splits are counted for the KV heads of a cache; all heads of a latent view share its rows, so it splits
+    keys by sequences and heads, and 32 sequences of 128 heads not at all."""
+    from types import SimpleNamespace
+
+    from easydel_b200.caching.paged import PagedBatchMeta, PagedLatentView
+
+    torch.manual_seed(0)
+    B, H, n = 32, 128, 700
+    rnd = lambda *s: (torch.randn(*s, device="cuda") * 0.3).to(torch.bfloat16)
+    mla = SimpleNamespace(kv_b_proj=SimpleNamespace(weight=rnd(H * 256, 512)), nope=128, vd=128, rope_dim=64, scale=0.07)
+    table = torch.arange(B * 32, dtype=torch.int32, device="cuda").view(B, 32)
+    view = PagedLatentView(rnd(B * 32, 128, 1, 576))
+    meta = PagedBatchMeta(cu_q=torch.arange(B + 1, dtype=torch.int32, device="cuda"),
+                          kv_lens=torch.full((B,), n, dtype=torch.int32, device="cuda"), page_table=table,
+                          slot_mapping=table[:, (n - 1) // 128] * 128 + (n - 1) % 128, max_q=1, num_seqs=B)
+    args = rnd(1, B, H, 128), rnd(1, B, H, 64), rnd(1, B, 512), rnd(1, B, 64)
+    got = []
+    for meta.num_splits in (1, 4):
+        got.append(view.attend_latent(mla, *args, meta))
+    assert torch.equal(*got)
+
+
 @pytest.mark.parametrize("B,H,n", [(32, 128, 600), (4, 128, 2000), (100, 64, 300)])
 def test_latent_decode_of_peaked_scores_keeps_the_output_s_precision(B, H, n):
     """Scores of a standard deviation of 2.25, so that a few keys carry most of a sum and maxima grow along a sequence: what is
