@@ -125,7 +125,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
   float* part = reinterpret_cast<float*>(smem);
   if (warp >= 2) {
     const int q = warp & 3, n = q * 32 + lane;
-    if (mbar_wait(b_done, 0, abort_flag, p.status, EDL_TIMEOUT_EPILOGUE)) {
+    if (__all_sync(0xffffffffu, mbar_wait(b_done, 0, abort_flag, p.status, EDL_TIMEOUT_EPILOGUE))) {
       tc_fence_after();
       for (int m0 = 0; m0 < p.M; m0 += 16) {
         uint32_t r[16];
