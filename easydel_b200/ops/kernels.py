@@ -40,8 +40,9 @@ def sm_count(device) -> int:
 def _splitk_plan(M: int, N: int, K: int, device) -> int:
     """Number of K slices for a skinny GEMM (1 = use the plain kernel).
 
-    Decode-time linears have a handful of rows and are bound by streaming the weight matrix; with one CTA per
-    128-column tile a 4096-wide projection would occupy 32 of 148 SMs. Slicing K gives every SM a share.
+    Decode-time linears have few rows and are bound by streaming the weight matrix; with one CTA per 128-column tile a
+    4096-wide projection would occupy 32 of 148 SMs. Slicing K gives every SM a share. What gets here has 129 to 256 rows, or
+    up to 128 and an output that the weight-streaming kernel (:func:`_skinny_plan`) does not take: not on 16 bytes.
     """
     if M > 256 or N % 8 or K % 64 or K < 512:
         return 1

@@ -130,12 +130,17 @@ def test_gemm_deterministic():
 
 
 @pytest.mark.parametrize("M,N,K", [(1, 4096, 4096), (16, 6144, 4096), (64, 1280, 8192), (256, 4096, 14336),
-                                   (48, 8192, 1024)])
-def test_gemm_skinny_uses_split_k(M, N, K):
-    """Decode-shaped products take the split-K path and agree with the fp32 reference (with and without bias)."""
+                                   (48, 8192, 1024), (129, 4096, 4096), (200, 1280, 8192)])
+def test_gemm_skinny_uses_split_k(M, N, K, monkeypatch):
+    """Decode-shaped products take the split-K path and agree with the fp32 reference (with and without bias). Up to 128 rows
+    that is the path of outputs the weight-streaming kernel does not take, which is put aside here."""
     from easydel_b200.ops import kernels as K_
 
     assert K_._splitk_plan(M, N, K, torch.device("cuda", 0)) > 1
+    calls, call = [], K_._lib.call
+    monkeypatch.setattr(K_._lib, "call", lambda name, *args: calls.append(name) or call(name, *args))
+    if M <= 128:
+        monkeypatch.setattr(K_, "_skinny_plan", lambda *args: 0)
     torch.manual_seed(M + N)
     a = torch.randn(M, K, device="cuda", dtype=torch.bfloat16)
     w = torch.randn(N, K, device="cuda", dtype=torch.bfloat16) * 0.05
@@ -145,6 +150,7 @@ def test_gemm_skinny_uses_split_k(M, N, K):
         ref = a.float() @ w.float().t() + (b.float() if b is not None else 0)
         err = (out.float() - ref).abs().max() / ref.abs().max()
         assert err < 1e-2, err
+    assert calls == ["edl_gemm_splitk"] * 2
 
 
 @pytest.mark.gpu
