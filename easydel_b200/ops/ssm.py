@@ -294,8 +294,9 @@ def ssd_scan_chunked(x, dt, A, B, C, D=None, dt_bias=None, softplus=True, cu_seq
 def ssd_scan(x, dt, A, B, C, D=None, dt_bias=None, softplus=True, cu_seqlens=None, state=None):
     """x ``[total, H, P]``; dt ``[total, H]``; A ``[H]``; B, C ``[total, G, N]``; state ``[nseq, H, P, N]`` fp32.
 
-    The kernels keep a workspace of 105 bytes per token and head, at most SCAN_WORKSPACE, besides 1680 per sequence and head.
-    A value that is not finite reaches outputs from its token on only."""
+    The kernels keep a workspace of 105 bytes per token and head, at most SCAN_WORKSPACE, besides 1680 per sequence and head;
+    where sequences are cut into segments, the states of about 1024 tiles of 64 columns too (33 MB for N = 128, twice that
+    with many sequences). A value that is not finite reaches outputs from its token on only."""
     if _use_kernel(x, dt, A, B, C, D) and B.shape[2] in (16, 32, 64, 128) and x.dtype == torch.bfloat16 \
             and x.shape[2] <= 256:
         total, H, P = x.shape
