@@ -9,6 +9,10 @@
     python -m benchmarks.profile_case ag_gemm       # one-rank form of the all-gather -> GEMM kernel
     python -m benchmarks.profile_case qgemv         # 4-bit fused dequant-GEMV, 4 rows x 14336 x 4096
     python -m benchmarks.profile_case qgemv_plain   # the same kernel as single launches (profiler captures)
+    python -m benchmarks.profile_case gemm_skinny   # 48 x 28672 x 4096: the weight-streaming product of a few rows
+    python -m benchmarks.profile_case delta         # gated delta rule, 5328 + 2864 tokens, 32 heads of 128 x 128
+    python -m benchmarks.profile_case ssd           # state-space scan, 3 x 2000 tokens, 64 heads of 64 x 128
+    python -m benchmarks.profile_case latent        # latent decode, 32 sequences of 2000 rows, 128 heads
     python -m benchmarks.profile_case adamw         # fused AdamW over 256M parameters
 
 Prints the CUDA-event time of the last launch. Everything held on the device stays below 4 GB.
@@ -105,6 +109,34 @@ def main() -> None:
             many()
         fn = g.replay
         work = graphed * (14336 * 4096 * 0.5 + 14336 * 64 * 2)     # bytes: the roofline of this kernel is HBM
+    elif what == "gemm_skinny":
+        a, w = bf(48, 4096), bf(28672, 4096)
+        out = torch.empty(48, 28672, device=dev, dtype=torch.bfloat16)
+        fn = lambda: K.gemm(a, w, out=out)  # noqa: E731
+        work = 2.0 * 28672 * 4096       # bytes of weights
+    elif what in ("delta", "ssd"):
+        from easydel_b200.ops import ssm
+
+        if what == "delta":
+            q, k = (torch.nn.functional.normalize(bf(8192, 32, 128), dim=-1) for _ in range(2))
+            v, g, beta = bf(8192, 32, 128), -torch.rand(8192, 32, device=dev), torch.rand(8192, 32, device=dev).bfloat16()
+            cu = torch.tensor([0, 5328, 8192], dtype=torch.int32, device=dev)
+            fn = lambda: ssm.gated_delta_rule(q, k, v, g, beta, None, cu)  # noqa: E731
+            work = 2.0 * 8192 * 32 * (4 * 128 + 1) + 4.0 * 8192 * 32
+        else:
+            x, dt, B, C = bf(6000, 64, 64), bf(6000, 64), bf(6000, 1, 128), bf(6000, 1, 128)
+            A, D = -torch.rand(64, device=dev) - 0.5, torch.randn(64, device=dev)
+            cu = torch.tensor([0, 2000, 4000, 6000], dtype=torch.int32, device=dev)
+            fn = lambda: ssm.ssd_scan(x, dt, A, B, C, D, None, True, cu)  # noqa: E731
+            work = 2.0 * 6000 * (64 * (2 * 64 + 1) + 2 * 128)
+    elif what == "latent":
+        from easydel_b200.ops import serving as S
+
+        pages, q = bf(32 * 16, 128, 1, 576), bf(32, 128, 576)
+        table = torch.arange(32 * 16, dtype=torch.int32, device=dev).view(32, 16)
+        lens = torch.full((32,), 2000, dtype=torch.int32, device=dev)
+        fn = lambda: S.mla_decode_attention(q, pages, lens, table, scale=0.07)  # noqa: E731
+        work = 2.0 * 32 * (2000 * 576 + 128 * (576 + 512))
     elif what == "adamw":
         n = 256 << 20
         p, g = torch.zeros(n, device=dev), torch.randn(n, device=dev)
@@ -124,7 +156,8 @@ def main() -> None:
     e1.record()
     torch.cuda.synchronize()
     ms = e0.elapsed_time(e1)
-    unit = "GB/s" if what in ("qgemv", "qgemv_plain", "adamw", "gemm_decode") else "TFLOP/s"
+    bound_by_bytes = ("qgemv", "qgemv_plain", "adamw", "gemm_decode", "gemm_skinny", "delta", "ssd", "latent")
+    unit = "GB/s" if what in bound_by_bytes else "TFLOP/s"
     rate = work / ms / 1e6 if unit == "GB/s" else work / ms / 1e9
     from easydel_b200.ops import _lib
 

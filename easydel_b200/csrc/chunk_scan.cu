@@ -22,11 +22,12 @@
 //   * chunk_scan: the columns of a state never meet. A warp owns 16 of them: S^T lies in the accumulator layout, which is also
 //     the layout of a left operand, so the state never leaves its registers; warps need no exchange. Rows, values and
 //     coefficients come by cp.async, two chunks ahead. What bounds it is the rate of the products: 168 of 16 x 8 x 16 per warp
-//     and chunk for the delta rule with DK = 128, 102 for the state space, at about 20 clocks each, and with one warp per
-//     scheduler the chain y -> T -> P behind them.
+//     and chunk for the delta rule with DK = 128, 102 for the state space, at about 20 clocks each (delta rule below, at most
+//     one warp per scheduler: 0.60 ms) and 23 per scheduler (second pass over the segments of the state space below: 0.20 ms),
+//     and with one warp per scheduler the chain y -> T -> P behind them.
 //
 // 5328 + 2864 tokens, 32 heads of 128 x 128: 0.64 ms (eight tokens at a time on the FMA pipe 1.90 ms, one at a time 19.4 ms);
-// 6000 tokens in three sequences, 64 state-space heads of 64 x 128: 0.30 ms (0.74 ms, 4.4 ms). Bytes at the copy rate: 43 and
+// 6000 tokens in three sequences, 64 state-space heads of 64 x 128: 0.32 ms (0.74 ms, 4.4 ms). Bytes at the copy rate: 43 and
 // 18 us. State-space sequences are cut into segments where that fills the GPU (cs_span): 8192 tokens of one sequence, 64 heads
 // 0.93 -> 0.38 ms, 8 heads 0.91 -> 0.09 ms. A value that is not finite reaches its column from its token on only, as in
 // a walk token by token: a chunk that holds one is summed on the FMA pipe (cs_triangle).
